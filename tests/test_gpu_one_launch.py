@@ -1,0 +1,101 @@
+"""GPU tests of the paths that a group of one rank takes when an op runs in one launch (the virtual-rank tests split every op
+into phases): rows that stay on the rank, against the CPU oracle, at the sizes where their loops end."""
+import pytest
+import torch
+
+import umdk_original_b200 as u
+from umdk_original_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+ops = torch.ops.umdk_cam_op_lib
+DEV = torch.device("cuda", 0)
+
+
+def _routing(t, e, k, seed, skip):
+    """Distinct experts per token where there are enough of them; every `skip`-th first choice is left out."""
+    g = torch.Generator().manual_seed(seed)
+    if e >= k:
+        idx = torch.rand(t, e, generator=g).argsort(dim=1)[:, :k].contiguous()
+    else:
+        idx = torch.randint(0, e, (t, k), generator=g)
+    if skip:
+        idx[::skip, 0] = -1
+    return idx, torch.rand(t, k, generator=g), g
+
+
+def _want(y, plan, idx, w, e, wire):
+    """Weighted sums of the rows y (receive order), in k order."""
+    if wire == 2:
+        y = ref.dequant_int8_1x128(*ref.quant_int8_1x128(y.float()))
+    t, k = idx.shape
+    rows = torch.zeros(t, k, y.shape[1])
+    rows[plan.src[:, 1].long(), plan.src[:, 2].long()] = y[:plan.src.shape[0]].float()
+    ok = ((idx >= 0) & (idx < e)).float().unsqueeze(-1)
+    acc = torch.zeros(t, y.shape[1])
+    for kk in range(k):
+        acc = torch.addcmul(acc, rows[:, kk] * ok[:, kk], w[:, kk].unsqueeze(-1))
+    return acc
+
+
+@pytest.mark.parametrize("t,h,e,k,skip", [(1, 128, 1, 1, 0), (3, 640, 6, 2, 2), (149, 1152, 10, 5, 7), (300, 512, 256, 8, 0),
+                                          (2500, 256, 601, 16, 3)])
+def test_prefill_pair_in_one_launch(t, h, e, k, skip):
+    # experts: one, not a multiple of four, more than the threads of a CTA (and odd); more pairs per CTA than threads at t = 2500
+    buf = u.Buffer(None, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, timeout_ms=2000.0), device=DEV, rank=0,
+                   num_ranks=1)
+    for it in range(2):  # the second call must not see the first one's rows
+        idx, w, g = _routing(t, e, k, seed=t + it, skip=skip if it == 0 else 0)
+        x = torch.randn(t, h, generator=g).to(torch.bfloat16)
+        plan = ref.plan_dispatch([idx], e)[0]
+        n = plan.src.shape[0]
+        rx, src, cnt, per_e, _ = ops.moe_dispatch_prefill_quant(x.to(DEV), idx.to(DEV), w.to(DEV), 0, buf.name, 0, 1, 0)
+        assert torch.equal(src.cpu().view(-1, 3), plan.src) and torch.equal(cnt.cpu(), plan.recv_count)
+        assert torch.equal(per_e.cpu(), plan.per_expert) and torch.equal(rx.cpu(), x[plan.src[:, 1].long()])
+        y = torch.randn(n, h, generator=g).to(torch.bfloat16)
+        out = ops.moe_combine_prefill(y.to(DEV), idx.to(DEV), w.to(DEV), src.clone(), cnt.clone(), buf.name, 0, 1)
+        buf.check()
+        want = _want(y, plan, idx, w, e, 0)
+        # the kernel adds the same products in the same order with fused multiply-adds; half a bf16 step remains
+        assert ((out.cpu().float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6 * k).all()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("quant,wire", [(0, 0), (2, 2), (3, 2), (4, 0)])
+@pytest.mark.parametrize("t,h,e,k,skip", [(1, 128, 1, 1, 0), (5, 1152, 6, 3, 2), (151, 512, 64, 8, 5), (256, 128, 8, 8, 0),
+                                          (257, 128, 16, 8, 3)])  # 2048 pairs: the most the scan of the ids serves
+def test_low_latency_pair_in_one_launch(t, h, e, k, skip, quant, wire):
+    buf = u.Buffer(None, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, ll_max_tokens=t, timeout_ms=2000.0),
+                   device=DEV, rank=0, num_ranks=1)
+    for it in range(2):
+        idx, w, g = _routing(t, e, k, seed=7 * t + it, skip=skip if it == 0 else 0)
+        idx = idx.to(torch.int32)
+        x = torch.randn(t, h, generator=g).to(torch.bfloat16)
+        smooth = torch.rand(e, h, generator=g) + 0.5 if quant == 2 else None
+        active = torch.arange(t) < t - t // 4
+        live = torch.where(active.unsqueeze(1), idx, torch.full_like(idx, -1))
+        plan = ref.plan_dispatch([live], e)[0]
+        n = plan.src.shape[0]
+        d = ops.moe_dispatch_shmem(x.to(DEV), idx.to(DEV), None if smooth is None else smooth.to(DEV), active.to(DEV), 1, 0, e,
+                                   1, 0, 0, 0, 0, quant, 0, it, buf.handle)
+        rows = x[plan.src[:, 1].long()]
+        if quant == 0:
+            assert torch.equal(d[0][:n].cpu(), rows)
+        elif quant == 2:
+            q, s = ref.quant_int8_token(rows.float() * smooth[live[plan.src[:, 1].long(), plan.src[:, 2].long()].long()])
+            assert (d[0][:n].cpu().int() - q.int()).abs().max() <= 1  # x * 127 / amax on a rounding boundary
+            assert torch.allclose(d[1][:n].cpu(), s, rtol=1e-6)
+        else:
+            q, s = ref.quant_fp8_1x128(rows, quant == 4)
+            assert torch.equal(d[0][:n].cpu().view(torch.uint8), q.view(torch.uint8)) and torch.equal(d[1][:n].cpu(), s)
+        assert torch.equal(d[2].cpu(), ref.slots_in_expert(live, e))
+        assert torch.equal(d[3].cpu(), plan.per_expert if it else plan.per_expert.cumsum(0))
+        assert torch.equal(d[4].cpu(), plan.recv_count) and d[5].tolist() == [0]
+        y = torch.randn(d[0].shape[0], h, generator=g).to(torch.bfloat16)
+        out = ops.moe_combine_shmem(y.to(DEV), idx.to(DEV), d[2], d[4], w.to(DEV), None, active.to(DEV), None, None, None, None,
+                                    1, 0, e, 1, 0, 0, 0, 0, 0, wire, buf.handle, 0, 0)
+        buf.check()
+        want = _want(y[:n], plan, live, w, e, wire)
+        # half a bf16 step; with int8 rows a value on a rounding boundary may also land one step (1 / 127 of its block) apart
+        slack = 1e-6 * k + (float(y.abs().max()) / 127 * float(w.max()) if wire else 0.0)
+        assert ((out.cpu().float() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
+    buf.destroy()

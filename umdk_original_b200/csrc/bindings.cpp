@@ -450,10 +450,9 @@ at::Tensor moe_combine_prefill_cuda(const at::Tensor& x, const at::Tensor& topk_
     const at::Tensor xk = rows_for_kernel(x, half, false);
     at::Tensor out = at::empty({T, h}, xk.options());
     // rows actually present: the smaller of x's rows and the device-side count of the last dispatch
-    at::Tensor total = at::minimum(b->total_recv(), at::full({1}, x.size(0), b->total_recv().options()));
-    CAM_RT(cam_combine(b->raw(), xk.data_ptr(), src_idx.data_ptr<int>(), total.data_ptr<int>(), topk_idx.data_ptr(),
-                       is64, w.data_ptr<float>(), out.data_ptr(), static_cast<int>(T), static_cast<int>(K),
-                       static_cast<int>(h), static_cast<int>(E), 0, 0,
+    CAM_RT(cam_combine(b->raw(), xk.data_ptr(), src_idx.data_ptr<int>(), cam_buffer_total_recv(b->raw()),
+                       static_cast<int>(x.size(0)), topk_idx.data_ptr(), is64, w.data_ptr<float>(), out.data_ptr(),
+                       static_cast<int>(T), static_cast<int>(K), static_cast<int>(h), static_cast<int>(E), 0, 0,
                        (g_phase_mask & 7) & (CAM_PHASE_SEND | CAM_PHASE_RECV), b->stream()));
     return half ? out.to(at::kHalf) : out;
 }
@@ -666,8 +665,8 @@ at::Tensor moe_combine_shmem_bf16(const at::Tensor& expandX, const at::Tensor& e
     at::Tensor out = at::empty({T, h}, expandX.options());
     if (g_phase_mask & 6)
     CAM_RT(cam_combine(b->raw(), y.data_ptr(), b->ll_src_.data_ptr<int>(), b->ll_total_.data_ptr<int>(),
-                       ids.data_ptr(), is64, w.data_ptr<float>(), out.data_ptr(), static_cast<int>(T),
-                       static_cast<int>(K), static_cast<int>(h), static_cast<int>(E), 1,
+                       static_cast<int>(std::min(b->ll_src_.size(0), y.size(0))), ids.data_ptr(), is64, w.data_ptr<float>(),
+                       out.data_ptr(), static_cast<int>(T), static_cast<int>(K), static_cast<int>(h), static_cast<int>(E), 1,
                        static_cast<int>(commQuantMode),
                        (g_phase_mask & 7) & (CAM_PHASE_SEND | CAM_PHASE_RECV), b->stream()));
     return out;

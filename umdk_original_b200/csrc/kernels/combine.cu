@@ -49,6 +49,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineParams p) {
     __shared__ uint32_t s_abort;
     __shared__ float s_w[kCombWarps][CAM_MAX_TOPK];
+    __shared__ uint64_t s_row[kCombWarps][CAM_MAX_TOPK];  // where the row of pair (t, k) is read from
     const int tid = static_cast<int>(threadIdx.x);
     const int warp = tid >> 5;
     const uint32_t lane = lane_id();
@@ -57,18 +58,39 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
     const int nwarps = nb * kCombWarps;
     const int row_bytes = p.h * 2;
     const uint32_t ep_send = p.epochs[0] + 1u, ep_recv = p.epochs[1] + 1u;
+    // Rows whose origin is this rank do not move when one launch sends and reduces: the send phase notes {epoch, row}
+    // per (token, k) pair, 8 bytes instead of a row written and read again, and the reduce gathers straight from y.
+    // The epoch tells this launch's entries from those of earlier ones.  A launch that runs one phase only (the fused
+    // layer's reduce, whose rows the GEMM epilogue has pushed, and the phase-by-phase harness) uses the slots.
+    // Bound by memory traffic: 4096 tokens x 8 rows of 14 KB on one GPU took 263 us with every row copied to its slot first
+    // (1.47 GB moved), 102 us with the rows gathered in place (0.53 GB, 5.2 TB/s).
+    const bool in_place = p.local_row != nullptr && p.y != nullptr &&
+                          (p.phase_mask & (CAM_PHASE_SEND | CAM_PHASE_RECV)) == (CAM_PHASE_SEND | CAM_PHASE_RECV);
     if (tid == 0) s_abort = 0u;
     __syncthreads();
 
     trace_point(p.trace, 0);  // kernel start
     // ------------------------------------------------------------------ SEND
     if (p.phase_mask & CAM_PHASE_SEND) {
-        const int n = p.total_rows[0];
+        const int n = min(p.total_rows[0], p.max_rows);
+        if (in_place) {  // one thread per row
+            for (int i = static_cast<int>(blockIdx.x) * kCombThreads + tid; i < n; i += nb * kCombThreads) {
+                const int src = p.row_src[static_cast<size_t>(i) * 3 + 0];
+                const int t = p.row_src[static_cast<size_t>(i) * 3 + 1];
+                const int k = p.row_src[static_cast<size_t>(i) * 3 + 2];
+                if (src < 0 || src >= p.R || t < 0 || t >= p.max_tokens || k < 0 || k >= p.K)
+                    comb_record_status(p.status, CAM_ERR_BAD_INDEX, 1, i);
+                else if (src == p.rank)
+                    p.local_row[static_cast<size_t>(t) * p.K + k] =
+                        (static_cast<uint64_t>(ep_send) << 32) | static_cast<uint32_t>(i);
+            }
+        }
         // Rows are ordered by expert and, inside an expert, by origin rank.  Every rank starts its walk somewhere else
         // (its share of the rows plus one grid-wide step per rank further on), so that at any one time the ranks of the
         // group push to different origins instead of all filling the same GPU's ingress.
         const int shift = (p.R > 1 && n > 0) ? static_cast<int>((static_cast<long long>(p.rank) * (n / p.R + nwarps)) % n) : 0;
-        for (int i0 = gwarp; i0 < n; i0 += nwarps) {
+        const int n_push = (in_place && p.R == 1) ? 0 : n;
+        for (int i0 = gwarp; i0 < n_push; i0 += nwarps) {
             const int i = (i0 + shift < n) ? i0 + shift : i0 + shift - n;
             const int src = p.row_src[static_cast<size_t>(i) * 3 + 0];
             const int t = p.row_src[static_cast<size_t>(i) * 3 + 1];
@@ -78,6 +100,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                 if (lane == 0) comb_record_status(p.status, CAM_ERR_BAD_INDEX, 1, i);
                 continue;
             }
+            if (in_place && src == p.rank) continue;
             const uint8_t* s = reinterpret_cast<const uint8_t*>(p.y) + static_cast<size_t>(i) * row_bytes;
             uint8_t* d = p.peer_base[src] + p.off_combine_buf +
                          (static_cast<size_t>(t) * p.K + k) * static_cast<size_t>(row_bytes);
@@ -169,6 +192,30 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
         if (s_abort) goto done;
 
         const uint8_t* buf = my_base + p.off_combine_buf;
+        // Weight, source address and presence of the pairs of token t, for this warp; bit k of the result: pair has a row.
+        // Bit 0 of an address (rows are 16-byte aligned) marks a row of y.
+        auto load_pairs = [&](int t) -> uint32_t {
+            bool pair_ok = false;
+            if (lane < static_cast<uint32_t>(p.K)) {
+                const size_t g = static_cast<size_t>(t) * p.K + lane;
+                const int id = load_expert_id(p.topk_idx, p.idx_is_i64, g);
+                s_w[warp][lane] = p.topk_weights[g];
+                uint64_t from = reinterpret_cast<uint64_t>(buf + g * row_bytes);
+                if (in_place) {
+                    const uint64_t ent = __ldcg(reinterpret_cast<const unsigned long long*>(p.local_row) + g);
+                    const bool here = static_cast<uint32_t>(ent >> 32) == ep_send;
+                    if (!here && p.R == 1) from = 0ull;  // no row of this call names the pair, and none can come from elsewhere
+                    if (here)
+                        from = (reinterpret_cast<uint64_t>(p.y) +
+                                static_cast<uint64_t>(static_cast<uint32_t>(ent)) * static_cast<uint64_t>(row_bytes)) | 1ull;
+                }
+                s_row[warp][lane] = from;
+                pair_ok = (id >= 0 && id < p.E && from != 0ull);
+            }
+            const uint32_t valid = __ballot_sync(0xFFFFFFFFu, pair_ok);
+            __syncwarp();
+            return valid;
+        };
         if (p.comm_quant == 2) {
             // rows arrived as int8 + one scale per 128 elements; a lane reduces 16 elements per step
             const int chunks_q = (p.h + 511) / 512;
@@ -178,15 +225,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                 const int t = it / nsplit_q;
                 const int e_begin = (it - t * nsplit_q) * per_q * 512;
                 const int e_end = min(p.h, e_begin + per_q * 512);
-                bool pair_ok = false;
-                if (lane < static_cast<uint32_t>(p.K)) {
-                    const int id = load_expert_id(p.topk_idx, p.idx_is_i64, static_cast<size_t>(t) * p.K + lane);
-                    s_w[warp][lane] = p.topk_weights[static_cast<size_t>(t) * p.K + lane];
-                    pair_ok = (id >= 0 && id < p.E);
-                }
-                const uint32_t valid = __ballot_sync(0xFFFFFFFFu, pair_ok);
-                __syncwarp();
-                const uint8_t* trow = buf + static_cast<size_t>(t) * p.K * row_bytes;
+                const uint32_t valid = load_pairs(t);
                 uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(t) * row_bytes;
                 for (int c = e_begin + static_cast<int>(lane) * 16; c < e_end; c += 512) {
                     float acc[16];
@@ -194,7 +233,32 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                     for (int j = 0; j < 16; ++j) acc[j] = 0.f;
                     for (int k = 0; k < p.K; ++k) {
                         if (!((valid >> k) & 1u)) continue;
-                        const uint8_t* krow = trow + static_cast<size_t>(k) * row_bytes;
+                        const uint64_t from = s_row[warp][k];
+                        if (from & 1ull) {
+                            // a row of y: quantised to the wire format here (8 lanes hold a 128-element block), so that
+                            // a row counts the same whether it travelled or not
+                            const uint8_t* yrow = reinterpret_cast<const uint8_t*>(from & ~1ull) + static_cast<size_t>(c) * 2;
+                            const uint4 y0 = ld_cg_v4(yrow), y1 = ld_cg_v4(yrow + 16);
+                            const float f[16] = {bf16_lo(y0.x), bf16_hi(y0.x), bf16_lo(y0.y), bf16_hi(y0.y),
+                                                 bf16_lo(y0.z), bf16_hi(y0.z), bf16_lo(y0.w), bf16_hi(y0.w),
+                                                 bf16_lo(y1.x), bf16_hi(y1.x), bf16_lo(y1.y), bf16_hi(y1.y),
+                                                 bf16_lo(y1.z), bf16_hi(y1.z), bf16_lo(y1.w), bf16_hi(y1.w)};
+                            float amax = 0.f;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+                            const uint32_t group = 0xFFu << (lane & 24u);  // h is a multiple of 128: all 8 lanes are here
+#pragma unroll
+                            for (int sft = 4; sft >= 1; sft >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, sft));
+                            const float a = fmaxf(amax, 1e-12f);
+                            const float inv = 127.f / a;
+                            const float sc = (a / 127.f) * s_w[warp][k];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                acc[j] = fmaf(sc, static_cast<float>(static_cast<int>(static_cast<int8_t>(
+                                                      static_cast<uint32_t>(__float2int_rn(f[j] * inv)) & 0xFFu))), acc[j]);
+                            continue;
+                        }
+                        const uint8_t* krow = reinterpret_cast<const uint8_t*>(from);
                         const uint4 q = ld_cg_v4(krow + c);
                         const float sc = __ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7)) * s_w[warp][k];
                         const uint32_t wq[4] = {q.x, q.y, q.z, q.w};
@@ -225,15 +289,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
             const int t = it / nsplit;
             const int o_begin = (it - t * nsplit) * per * 512;
             const int o_end = min(row_bytes, o_begin + per * 512);
-            bool pair_ok = false;
-            if (lane < static_cast<uint32_t>(p.K)) {
-                const int id = load_expert_id(p.topk_idx, p.idx_is_i64, static_cast<size_t>(t) * p.K + lane);
-                s_w[warp][lane] = p.topk_weights[static_cast<size_t>(t) * p.K + lane];
-                pair_ok = (id >= 0 && id < p.E);
-            }
-            const uint32_t valid = __ballot_sync(0xFFFFFFFFu, pair_ok);  // bit k: pair (t, k) has a row
-            __syncwarp();
-            const uint8_t* trow = buf + static_cast<size_t>(t) * p.K * row_bytes;
+            const uint32_t valid = load_pairs(t);
             uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(t) * row_bytes;
             for (int o = o_begin + static_cast<int>(lane) * 16; o < o_end; o += 512) {
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -243,7 +299,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                     for (int j = 0; j < 8; ++j) {
                         const int k = k0 + j;
                         const bool ok = (k < p.K) && ((valid >> k) & 1u);
-                        v[j] = ok ? ld_cg_v4(trow + static_cast<size_t>(k) * row_bytes + o) : make_uint4(0, 0, 0, 0);
+                        v[j] = ok ? ld_cg_v4(reinterpret_cast<const uint8_t*>(s_row[warp][k] & ~1ull) + o) : make_uint4(0, 0, 0, 0);
                     }
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {

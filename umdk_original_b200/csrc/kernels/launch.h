@@ -65,6 +65,7 @@ struct CombineParams {
     const __nv_bfloat16* y;   // [N, h] expert outputs in receive order (SEND phase)
     const int* row_src;       // [N, 3] (src rank, src token, src k)
     const int* total_rows;    // [1] device-side N
+    int max_rows;             // rows y holds: N is never taken larger
     const void* topk_idx;     // [T, K] of this rank's own tokens (RECV phase)
     int idx_is_i64;
     const float* topk_weights;  // [T, K]
@@ -83,6 +84,7 @@ struct CombineParams {
     unsigned int* done_ctr;
     CamStatus* status;
     CamStatsDev* stats;  // optional
+    uint64_t* local_row;  // [max_tokens * K] {epoch, row of y} of the pairs whose rows stay on this rank (null: none do)
 };
 
 struct DispatchLLParams {

@@ -48,6 +48,10 @@ uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
 // Floats between two rows of activation scales on the deep-fused route: the fused kernel reads a row four K-blocks
 // (16 bytes) at a time.
 uint64_t scale_row_pitch(uint64_t blocks) { return align_up(blocks, 4); }
+// Bytes of the two {epoch, row} tables of combine (normal and low-latency; their epochs count separately).
+size_t local_row_bytes(const CamLayout& L) {
+    return sizeof(uint64_t) * (static_cast<size_t>(L.max_tokens) + L.ll_max_tokens) * L.topk;
+}
 
 }  // namespace
 
@@ -73,6 +77,7 @@ struct CamBuffer {
     int* num_tokens_per_expert = nullptr;
     unsigned int* done_ctr = nullptr;  // [4]: dispatch, combine, gemm, spare
     unsigned int* dup_ctr = nullptr;   // [CAM_MAX_RANKS] replicate-list cursors of normal dispatch (self-resetting)
+    uint64_t* local_row = nullptr;     // combine's {epoch, row} per pair: [max_tokens * topk] normal, then low latency
     CamStatus* d_status = nullptr;
     CamStatus* h_status = nullptr;  // pinned
     uint8_t* act_q = nullptr;       // [capacity, hidden] scratch between the two GEMMs (sized for I <= hidden)
@@ -259,6 +264,7 @@ extern "C" CamBuffer* cam_buffer_create(int device, int rank, int num_ranks, con
     ok &= cudaMalloc(&b->num_tokens_per_expert, sizeof(int) * E) == cudaSuccess;
     ok &= cudaMalloc(&b->done_ctr, sizeof(unsigned int) * 4) == cudaSuccess;
     ok &= cudaMalloc(&b->dup_ctr, sizeof(unsigned int) * CAM_MAX_RANKS) == cudaSuccess;
+    ok &= cudaMalloc(&b->local_row, local_row_bytes(*layout)) == cudaSuccess;
     ok &= cudaMalloc(&b->d_epochs, sizeof(uint32_t) * 16) == cudaSuccess;
     ok &= cudaMalloc(&b->exit_ctr, sizeof(unsigned int) * 4) == cudaSuccess;
     ok &= cudaMalloc(&b->d_status, sizeof(CamStatus)) == cudaSuccess;
@@ -274,6 +280,7 @@ extern "C" CamBuffer* cam_buffer_create(int device, int rank, int num_ranks, con
     cudaMemset(b->d_stats, 0, sizeof(cam::CamStatsDev));
     cudaMemset(b->done_ctr, 0, sizeof(unsigned int) * 4);
     cudaMemset(b->dup_ctr, 0, sizeof(unsigned int) * CAM_MAX_RANKS);
+    cudaMemset(b->local_row, 0, local_row_bytes(*layout));  // epoch 0 is never used
     cudaMemset(b->d_epochs, 0, sizeof(uint32_t) * 16);
     cudaMemset(b->exit_ctr, 0, sizeof(unsigned int) * 4);
     cudaMemset(b->d_status, 0, sizeof(CamStatus));
@@ -294,7 +301,7 @@ extern "C" int cam_buffer_destroy(CamBuffer* b) {
     if (b->tp_peer != nullptr && b->tp_peer_is_ipc) cudaIpcCloseMemHandle(b->tp_peer);
     void* frees[] = {b->base, b->d_peer_table, b->cta_hist, b->slot_in_expert, b->send_row, b->recv_count,
                      b->expert_offsets, b->num_recv_per_expert, b->total_recv, b->num_tokens_per_expert,
-                     b->done_ctr, b->dup_ctr, b->d_epochs, b->exit_ctr, b->d_status, b->act_q, b->act_s};
+                     b->done_ctr, b->dup_ctr, b->local_row, b->d_epochs, b->exit_ctr, b->d_status, b->act_q, b->act_s};
     for (void* p : frees)
         if (p != nullptr) cudaFree(p);
     if (b->h_status != nullptr) cudaFreeHost(b->h_status);
@@ -363,6 +370,7 @@ extern "C" int cam_buffer_reset(CamBuffer* b, cudaStream_t stream) {
     CAM_CUDA(cudaMemsetAsync(b->base, 0, b->layout.off_recv_x, stream));
     CAM_CUDA(cudaMemsetAsync(b->done_ctr, 0, sizeof(unsigned int) * 4, stream));
     CAM_CUDA(cudaMemsetAsync(b->dup_ctr, 0, sizeof(unsigned int) * CAM_MAX_RANKS, stream));
+    CAM_CUDA(cudaMemsetAsync(b->local_row, 0, local_row_bytes(b->layout), stream));  // epochs start again at 1
     CAM_CUDA(cudaMemsetAsync(b->d_epochs, 0, sizeof(uint32_t) * 16, stream));
     CAM_CUDA(cudaMemsetAsync(b->exit_ctr, 0, sizeof(unsigned int) * 4, stream));
     CAM_CUDA(cudaMemsetAsync(b->d_status, 0, sizeof(CamStatus), stream));
@@ -756,7 +764,7 @@ extern "C" int cam_dispatch_normal(CamBuffer* b, const void* x, const void* topk
     return dispatch_normal_impl(b, x, topk_idx, idx_is_i64, T, K, h, E, quant_mode, phase_mask, false, stream);
 }
 
-extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, const int* total_rows,
+extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, const int* total_rows, int max_rows,
                            const void* topk_idx, int idx_is_i64, const float* topk_weights, void* out, int T, int K,
                            int h, int E, int low_latency, int comm_quant, int phase_mask, cudaStream_t stream) {
     if (check_common(b, T, K, h, E, "combine") != 0) return -1;
@@ -768,6 +776,7 @@ extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, cons
     p.y = static_cast<const __nv_bfloat16*>(y);
     p.row_src = row_src;
     p.total_rows = total_rows;
+    p.max_rows = max_rows;
     p.topk_idx = topk_idx;
     p.idx_is_i64 = idx_is_i64;
     p.topk_weights = topk_weights;
@@ -787,6 +796,7 @@ extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, cons
     p.done_ctr = b->done_ctr + 1;
     p.status = b->d_status;
     p.stats = low_latency ? nullptr : b->d_stats;
+    p.local_row = b->local_row + (low_latency ? static_cast<size_t>(b->layout.max_tokens) * b->layout.topk : 0);
     const int rc = cam_launch_combine(&p, b->num_sms, stream);
     CAM_CHECK(rc == 0, "combine launch failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
     if (b != nullptr) ++b->launches;
@@ -1172,7 +1182,7 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
     }
     stamp(3);
     if (phase_mask & 8) {
-        if (cam_combine(b, nullptr, nullptr, nullptr, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
+        if (cam_combine(b, nullptr, nullptr, nullptr, 0, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
                         CAM_PHASE_RECV, stream) != 0)
             return -1;
     }
@@ -1274,7 +1284,7 @@ static int fused_moe_deep(CamBuffer* b, const void* x, const void* expert_ids, i
     stamp(2);
     stamp(3);
     if (phase_mask & 8) {
-        if (cam_combine(b, nullptr, nullptr, nullptr, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
+        if (cam_combine(b, nullptr, nullptr, nullptr, 0, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
                         CAM_PHASE_RECV, stream) != 0)
             return -1;
     }
@@ -1349,7 +1359,7 @@ static int fused_moe_impl(CamBuffer* b, const void* x, const void* expert_ids, i
     }
     stamp(3);
     if (phase_mask & 8) {
-        if (cam_combine(b, nullptr, nullptr, nullptr, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
+        if (cam_combine(b, nullptr, nullptr, nullptr, 0, expert_ids, idx_is_i64, topk_weights, out, T, K, h, E, 0, 0,
                         CAM_PHASE_RECV, stream) != 0)
             return -1;
     }

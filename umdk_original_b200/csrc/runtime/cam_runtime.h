@@ -104,8 +104,9 @@ int cam_dispatch_normal(CamBuffer* b, const void* x_bf16, const void* topk_idx, 
 // Combine (push + flag + weighted reduce).  `y` rows follow `row_src` ([N,3] device ints), N is
 // read on the device from `total_rows`.  low_latency selects the low-latency slot/flag regions.
 // comm_quant 2 sends rows as int8 with one fp32 scale per 128 elements (both phases of a call must agree).
-int cam_combine(CamBuffer* b, const void* y_bf16, const int* row_src, const int* total_rows, const void* topk_idx,
-                int idx_is_i64, const float* topk_weights, void* out_bf16, int T, int K, int h, int E,
+// max_rows bounds N (the rows y holds).
+int cam_combine(CamBuffer* b, const void* y_bf16, const int* row_src, const int* total_rows, int max_rows,
+                const void* topk_idx, int idx_is_i64, const float* topk_weights, void* out_bf16, int T, int K, int h, int E,
                 int low_latency, int comm_quant, int phase_mask, cudaStream_t stream);
 
 int cam_dispatch_ll(CamBuffer* b, const void* x_bf16, const void* expert_ids, int idx_is_i64, const float* smooth,
