@@ -507,6 +507,7 @@ std::vector<at::Tensor> moe_dispatch_shmem_bf16(const at::Tensor& x, const at::T
     at::Tensor smooth_t;
     if (scales.has_value() && scales->defined() && quantMode == 2) {
         smooth_t = scales->to(at::kFloat).contiguous();
+        if (reinterpret_cast<uintptr_t>(smooth_t.data_ptr()) & 7) smooth_t = smooth_t.clone();  // read 8 bytes at a time
         CAM_ASSERT(smooth_t.dim() == 2 && smooth_t.size(0) >= moeExpertNum && smooth_t.size(1) == h,
                    "scales must be [>= moeExpertNum, h]");
         CAM_ASSERT(S == 0, "smooth scales together with shared-expert ranks are not supported");
@@ -522,16 +523,20 @@ std::vector<at::Tensor> moe_dispatch_shmem_bf16(const at::Tensor& x, const at::T
     at::Tensor expandSrc = at::empty({A, 3}, x.options().dtype(at::kInt));
     at::Tensor tokenNums = at::empty({El}, x.options().dtype(at::kLong));
     at::Tensor epSend = at::empty({epWorldSize * El}, x.options().dtype(at::kInt));
-    at::Tensor tpSend = at::zeros({std::max<int64_t>(tpWorldSize, 1)}, x.options().dtype(at::kInt));
-    at::Tensor total = at::zeros({1}, x.options().dtype(at::kInt));
-    if (g_phase_mask & 6)
+    // the dispatch kernel sets these two; a call that runs none of its phases starts them here
+    const bool launches = (g_phase_mask & 6) != 0;
+    const auto iopt = x.options().dtype(at::kInt);
+    at::Tensor tpSend = launches ? at::empty({std::max<int64_t>(tpWorldSize, 1)}, iopt) : at::zeros({std::max<int64_t>(tpWorldSize, 1)}, iopt);
+    at::Tensor total = launches ? at::empty({1}, iopt) : at::zeros({1}, iopt);
+    if (launches)
     CAM_RT(cam_dispatch_ll(b->raw(), x.data_ptr(), ids.data_ptr(), is64, smooth, static_cast<int>(T),
                            static_cast<int>(K), static_cast<int>(h), static_cast<int>(E),
                            static_cast<int>(active), static_cast<int>(quantMode), static_cast<int>(expertTokenNumsType),
                            expandX.data_ptr(), dynScales.data_ptr<float>(), expandIdx.data_ptr<int>(),
                            expandSrc.data_ptr<int>(), tokenNums.data_ptr<int64_t>(), epSend.data_ptr<int>(),
-                           total.data_ptr<int>(), (g_phase_mask & 7) & (CAM_PHASE_SEND | CAM_PHASE_RECV), b->stream()));
-    if (g_phase_mask & 6) {
+                           total.data_ptr<int>(), tpSend.data_ptr<int>(), static_cast<int>(tpSend.numel()),
+                           (g_phase_mask & 7) & (CAM_PHASE_SEND | CAM_PHASE_RECV), b->stream()));
+    if (launches) {
         b->ll_src_ = expandSrc;
         b->ll_total_ = total;
     }

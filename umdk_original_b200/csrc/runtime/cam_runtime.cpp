@@ -807,7 +807,7 @@ extern "C" int cam_dispatch_ll(CamBuffer* b, const void* x, const void* expert_i
                                const float* smooth, int T, int K, int h, int E, int active_tokens, int quant_mode,
                                int count_type, void* expand_x, float* expand_scales, int* expand_idx,
                                int* expand_src, int64_t* expert_token_nums, int* ep_send_counts, int* total_rows,
-                               int phase_mask, cudaStream_t stream) {
+                               int* tp_zero, int tp_words, int phase_mask, cudaStream_t stream) {
     if (check_common(b, T, K, h, E, "dispatch_ll") != 0) return -1;
     CAM_CHECK(b->layout.ll_max_tokens > 0, "dispatch_ll: the buffer was created without low-latency regions");
     CAM_CHECK(T <= b->layout.ll_max_tokens, "dispatch_ll: %d tokens exceed ll_max_tokens %d", T, b->layout.ll_max_tokens);
@@ -845,6 +845,8 @@ extern "C" int cam_dispatch_ll(CamBuffer* b, const void* x, const void* expert_i
     p.expert_token_nums = expert_token_nums;
     p.ep_send_counts = ep_send_counts;
     p.total_rows = total_rows;
+    p.tp_zero = tp_zero;
+    p.tp_words = tp_words;
     p.status = b->d_status;
     int grid;
     const auto gkey = std::make_tuple(h, quant_mode, T, K);
@@ -856,9 +858,9 @@ extern "C" int cam_dispatch_ll(CamBuffer* b, const void* x, const void* expert_i
         b->ll_grid_cache[gkey] = grid;
     }
     CAM_CHECK(grid > 0, "dispatch_ll: kernel does not fit (shared memory for T=%d K=%d h=%d)", T, K, h);
-    // one token per CTA when sending, one row per warp when packing: no more CTAs than that needs
-    // (a smaller grid makes the grid-wide barrier cheaper)
-    int want = (T * K + 15) / 16;
+    // one token per CTA when sending (int8: one row per four warps), one row per warp when packing: no more CTAs than
+    // that needs (a smaller grid makes the grid-wide barrier cheaper)
+    int want = quant_mode == CAM_QUANT_INT8_TOKEN ? (T * K + 3) / 4 : (T * K + 15) / 16;
     if (want < T) want = T;
     if (want < 8) want = 8;
     if (grid > want) grid = want;
