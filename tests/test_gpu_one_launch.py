@@ -99,3 +99,12 @@ def test_low_latency_pair_in_one_launch(t, h, e, k, skip, quant, wire):
         slack = 1e-6 * k + (float(y.abs().max()) / 127 * float(w.max()) if wire else 0.0)
         assert ((out.cpu().float() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
     buf.destroy()
+
+
+@pytest.mark.parametrize("t,e,k,r", [(0, 8, 2, 2), (1, 1, 1, 1), (33, 72, 3, 72), (4097, 256, 8, 8), (16384, 64, 16, 4),
+                                     (16385, 64, 2, 64)])  # 16384 tokens: the most the one-launch form serves
+def test_layout_at_its_sizes(t, e, k, r):
+    idx = torch.randint(-1, e + 1, (t, k), generator=torch.Generator().manual_seed(t))
+    got = ops.get_dispatch_layout(idx.to(DEV), e, r)
+    for a, b in zip(got, ref.get_dispatch_layout(idx, e, r)):
+        assert torch.equal(a.cpu(), b)

@@ -344,9 +344,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> get_dispatch_layout_cuda(const at
     c10::cuda::CUDAGuard guard(topk_idx.device());
     const int64_t T = topk_idx.size(0), K = topk_idx.size(1);
     auto opts = topk_idx.options().dtype(at::kInt);
-    at::Tensor per_rank = at::zeros({num_ranks}, opts);
-    at::Tensor per_expert = at::zeros({num_experts}, opts);
-    at::Tensor in_rank = at::zeros({T, num_ranks}, topk_idx.options().dtype(at::kBool));
+    at::Tensor per_rank = at::empty({num_ranks}, opts);
+    at::Tensor per_expert = at::empty({num_experts}, opts);
+    at::Tensor in_rank = at::empty({T, num_ranks}, topk_idx.options().dtype(at::kBool));
     CAM_RT(cam_get_dispatch_layout(topk_idx.data_ptr(), is64, static_cast<int>(T), static_cast<int>(K),
                                    static_cast<int>(num_experts), static_cast<int>(num_ranks),
                                    per_rank.data_ptr<int>(), per_expert.data_ptr<int>(),

@@ -91,7 +91,7 @@ int cam_buffer_barrier(CamBuffer* b, int phase_mask, cudaStream_t stream);
 int cam_buffer_p2p_write(CamBuffer* b, int peer, size_t bytes, int grid, cudaStream_t stream);
 int cam_buffer_p2p_pingpong(CamBuffer* b, int peer, unsigned int base, int iters, int initiator, cudaStream_t stream);
 
-// get_dispatch_layout: outputs must be zero-initialised by the caller.
+// get_dispatch_layout: writes every element of its outputs.
 int cam_get_dispatch_layout(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R,
                             int* num_tokens_per_rank, int* num_tokens_per_expert, uint8_t* is_token_in_rank,
                             cudaStream_t stream);
