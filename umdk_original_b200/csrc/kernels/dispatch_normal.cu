@@ -460,6 +460,55 @@ __global__ void layout_kernel(const void* topk_idx, int idx_is_i64, int T, int K
     for (int i = threadIdx.x; i < E; i += blockDim.x) if (s_exp[i]) atomicAdd(&num_tokens_per_expert[i], s_exp[i]);
 }
 
+// The same in ONE launch without zeroed outputs, for batches of ordinary size: a cluster of kLayoutCtas CTAs counts in
+// shared memory, and after a cluster barrier every CTA adds up its share of the counters over the cluster's shared memories.
+// The call is bound by launches (about 3 us of host time each), not by the 64 bytes per token it reads: the counting kernel
+// above needs its three outputs zeroed first.  Up to kLayoutClusterTokens (four tokens per thread) the few CTAs cost less
+// than those launches; beyond, the whole GPU counts.  4096 tokens x 8: 22.5 us -> 9.6 us per call.
+constexpr int kLayoutCtas = 8, kLayoutThreads = 512, kLayoutClusterTokens = 4 * kLayoutCtas * kLayoutThreads;
+
+__global__ void __cluster_dims__(kLayoutCtas, 1, 1) __launch_bounds__(kLayoutThreads)
+layout_cluster_kernel(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R, int* num_tokens_per_rank,
+                      int* num_tokens_per_expert, uint8_t* is_token_in_rank) {
+    __shared__ int s_cnt[CAM_MAX_EXPERTS + CAM_MAX_RANKS];  // per expert, then per rank
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = static_cast<int>(threadIdx.x), rank = static_cast<int>(cluster.block_rank());
+    const int n = E + R, El = E / R;
+    for (int i = tid; i < n; i += kLayoutThreads) s_cnt[i] = 0;
+    __syncthreads();
+    for (int tb = rank * kLayoutThreads + (tid & ~31); tb < T; tb += kLayoutCtas * kLayoutThreads) {
+        const int t = tb + (tid & 31);  // whole warps stay together: the last one may hold lanes past T
+        unsigned long long seen_lo = 0ull, seen_hi = 0ull;  // ranks 0..63 and 64..127
+        for (int k0 = 0; k0 < K; k0 += 8) {                 // eight loads in flight
+            int id[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                id[j] = (t < T && k0 + j < K) ? load_expert_id(topk_idx, idx_is_i64, static_cast<size_t>(t) * K + k0 + j) : -1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (id[j] < 0 || id[j] >= E) continue;
+                atomicAdd(&s_cnt[id[j]], 1);
+                const int r = id[j] / El;
+                if (r < 64) seen_lo |= 1ull << r; else seen_hi |= 1ull << (r - 64);
+            }
+        }
+        for (int r = 0; r < R; ++r) {
+            const bool in = (r < 64) ? ((seen_lo >> r) & 1ull) : ((seen_hi >> (r - 64)) & 1ull);
+            if (t < T) is_token_in_rank[static_cast<size_t>(t) * R + r] = in ? 1 : 0;
+            const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);  // one atomic per warp: few ranks, many tokens
+            if ((tid & 31) == 0 && all != 0u) atomicAdd(&s_cnt[E + r], __popc(all));
+        }
+    }
+    cluster.sync();
+    for (int i = rank * kLayoutThreads + tid; i < n; i += kLayoutCtas * kLayoutThreads) {
+        int sum = 0;
+#pragma unroll
+        for (int c = 0; c < kLayoutCtas; ++c) sum += cluster.map_shared_rank(s_cnt, c)[i];
+        if (i < E) num_tokens_per_expert[i] = sum; else num_tokens_per_rank[i - E] = sum;
+    }
+    cluster.sync();  // no CTA leaves while others read its counters
+}
+
 }  // namespace cam
 
 // ----------------------------------------------------------------------------------------
@@ -512,52 +561,3 @@ extern "C" int cam_launch_layout(const void* topk_idx, int idx_is_i64, int T, in
                                                        num_tokens_per_expert, is_token_in_rank);
     return static_cast<int>(cudaGetLastError());
 }
-// The same in ONE launch without zeroed outputs, for batches of ordinary size: a cluster of kLayoutCtas CTAs counts in
-// shared memory, and after a cluster barrier every CTA adds up its share of the counters over the cluster's shared memories.
-// The call is bound by launches (about 3 us of host time each), not by the 64 bytes per token it reads: the counting kernel
-// above needs its three outputs zeroed first.  Up to kLayoutClusterTokens (four tokens per thread) the few CTAs cost less
-// than those launches; beyond, the whole GPU counts.  4096 tokens x 8: 22.5 us -> 9.6 us per call.
-constexpr int kLayoutCtas = 8, kLayoutThreads = 512, kLayoutClusterTokens = 4 * kLayoutCtas * kLayoutThreads;
-
-__global__ void __cluster_dims__(kLayoutCtas, 1, 1) __launch_bounds__(kLayoutThreads)
-layout_cluster_kernel(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R, int* num_tokens_per_rank,
-                      int* num_tokens_per_expert, uint8_t* is_token_in_rank) {
-    __shared__ int s_cnt[CAM_MAX_EXPERTS + CAM_MAX_RANKS];  // per expert, then per rank
-    cg::cluster_group cluster = cg::this_cluster();
-    const int tid = static_cast<int>(threadIdx.x), rank = static_cast<int>(cluster.block_rank());
-    const int n = E + R, El = E / R;
-    for (int i = tid; i < n; i += kLayoutThreads) s_cnt[i] = 0;
-    __syncthreads();
-    for (int tb = rank * kLayoutThreads + (tid & ~31); tb < T; tb += kLayoutCtas * kLayoutThreads) {
-        const int t = tb + (tid & 31);  // whole warps stay together: the last one may hold lanes past T
-        unsigned long long seen_lo = 0ull, seen_hi = 0ull;  // ranks 0..63 and 64..127
-        for (int k0 = 0; k0 < K; k0 += 8) {                 // eight loads in flight
-            int id[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                id[j] = (t < T && k0 + j < K) ? load_expert_id(topk_idx, idx_is_i64, static_cast<size_t>(t) * K + k0 + j) : -1;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (id[j] < 0 || id[j] >= E) continue;
-                atomicAdd(&s_cnt[id[j]], 1);
-                const int r = id[j] / El;
-                if (r < 64) seen_lo |= 1ull << r; else seen_hi |= 1ull << (r - 64);
-            }
-        }
-        for (int r = 0; r < R; ++r) {
-            const bool in = (r < 64) ? ((seen_lo >> r) & 1ull) : ((seen_hi >> (r - 64)) & 1ull);
-            if (t < T) is_token_in_rank[static_cast<size_t>(t) * R + r] = in ? 1 : 0;
-            const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);  // one atomic per warp: few ranks, many tokens
-            if ((tid & 31) == 0 && all != 0u) atomicAdd(&s_cnt[E + r], __popc(all));
-        }
-    }
-    cluster.sync();
-    for (int i = rank * kLayoutThreads + tid; i < n; i += kLayoutCtas * kLayoutThreads) {
-        int sum = 0;
-#pragma unroll
-        for (int c = 0; c < kLayoutCtas; ++c) sum += cluster.map_shared_rank(s_cnt, c)[i];
-        if (i < E) num_tokens_per_expert[i] = sum; else num_tokens_per_rank[i - E] = sum;
-    }
-    cluster.sync();  // no CTA leaves while others read its counters
-}
-
