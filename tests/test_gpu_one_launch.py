@@ -108,3 +108,36 @@ def test_layout_at_its_sizes(t, e, k, r):
     got = ops.get_dispatch_layout(idx.to(DEV), e, r)
     for a, b in zip(got, ref.get_dispatch_layout(idx, e, r)):
         assert torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("quant", [0, 2, 3, 4])
+@pytest.mark.parametrize("t,h,e,k", [(1, 128, 1, 1), (149, 1408, 5, 3), (512, 256, 32, 8), (513, 256, 32, 8), (592, 384, 7, 2),
+                                     (593, 384, 7, 2)])  # 4096 pairs and four tokens per CTA: the most the short form serves
+def test_prefill_dispatch_formats_in_one_launch(t, h, e, k, quant):
+    buf = u.Buffer(None, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, timeout_ms=2000.0), device=DEV, rank=0,
+                   num_ranks=1)
+    idx, w, g = _routing(t, e, k, seed=3 * t + quant, skip=4)
+    x = torch.randn(t, h, generator=g).to(torch.bfloat16)
+    plan = ref.plan_dispatch([idx], e)[0]
+    n = plan.src.shape[0]
+    if n == 0:  # the only pair is the one left out
+        idx[0, 0] = 0
+        plan = ref.plan_dispatch([idx], e)[0]
+        n = 1
+    rx, src, cnt, per_e, rs = ops.moe_dispatch_prefill_quant(x.to(DEV), idx.to(DEV), w.to(DEV), buf.capacity, buf.name, 0, 1, quant)
+    buf.check()
+    rows = x[plan.src[:, 1].long()]
+    assert torch.equal(src.cpu().view(-1, 3)[:n], plan.src) and torch.equal(cnt.cpu(), plan.recv_count)
+    assert torch.equal(per_e.cpu(), plan.per_expert) and int(buf.native.total_recv()) == n
+    if quant == 0:
+        assert torch.equal(rx[:n].cpu(), rows)
+    elif quant == 2:
+        q, s = ref.quant_int8_token(rows)
+        assert (rx[:n].cpu().int() - q.int()).abs().max() <= 1  # x * 127 / amax on a rounding boundary
+        assert torch.allclose(rs[:n].cpu().reshape(-1), s, rtol=1e-6)
+    else:
+        q, s = ref.quant_fp8_1x128(rows, quant == 4)
+        assert torch.equal(rx[:n].cpu().view(torch.uint8), q.view(torch.uint8)) and torch.equal(rs[:n].cpu(), s)
+    stats = buf.stats()
+    assert stats["dispatch_calls"] == 1 and stats["rows_routed_to_peer"] == [n]
+    buf.destroy()

@@ -788,7 +788,9 @@ std::vector<at::Tensor> fused_deep_moe_bf16(const at::Tensor& x, const at::Tenso
     const int is64 = idx_kind(ids, "expertIds");
     const int64_t K = ids.size(1);
     at::Tensor out = at::empty({T, h}, x.options());
-    at::Tensor nums = at::zeros({El}, x.options().dtype(at::kLong));
+    // written by the receive phase; a call that does not run it (one phase of the test harness) returns zeros
+    const auto lopt = x.options().dtype(at::kLong);
+    at::Tensor nums = (g_phase_mask & CAM_PHASE_RECV) ? at::empty({El}, lopt) : at::zeros({El}, lopt);
     auto fused = w8a8 ? &cam_fused_moe_w8a8 : quantMode == 4 ? &cam_fused_moe_mxfp8 : &cam_fused_moe_fp8;
     const void* w1p = w8a8 ? w1k.data_ptr() : w1.data_ptr();
     const void* w2p = w8a8 ? w2k.data_ptr() : w2.data_ptr();

@@ -70,18 +70,20 @@ __device__ __forceinline__ void warp_quant_fp8_1x128(const __nv_bfloat16* __rest
                                                      uint8_t* q, float* s) {
     const uint32_t lane = lane_id();
     // Each lane owns 8 consecutive elements per step of 256; 16 lanes cover one 128-element block.
-    // The loads of four steps are issued together (the steps are independent), which divides the
-    // number of exposed memory latencies per row by four.
-    for (int base = 0; base < h; base += 1024) {
-        uint4 v[4];
+    // The loads of eight steps are issued together (the steps are independent), which divides the
+    // number of exposed memory latencies per row by eight.
+    constexpr int U = 8;
+    for (int base = 0; base < h; base += U * 256) {
+        uint4 v[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int c = base + u * 256 + static_cast<int>(lane) * 8;
             v[u] = (c < h) ? ld_nc_v4(row + c) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int c = base + u * 256 + static_cast<int>(lane) * 8;
+            if (c - static_cast<int>(lane) * 8 >= h) break;  // the same in all lanes
             float sc;
             const uint2 o2 = quant8_in_block16<UE8M0>(v[u], sc);
             if (c < h) {

@@ -16,6 +16,7 @@
 #include "../common/cam_types.h"
 #include "../common/ptx.cuh"
 #include "../common/quant.cuh"
+#include "../common/slots.cuh"
 #include "launch.h"
 
 namespace cg = cooperative_groups;
@@ -24,6 +25,11 @@ namespace cam {
 
 constexpr int kDispThreads = 512;
 constexpr int kDispWarps = kDispThreads / 32;
+constexpr int kDispGroups = 16;  // most runs of rows that the column sums of the count phase are cut into
+// Count-phase tables in dynamic shared memory: warp x expert counts, later the partial column sums (2 x groups x E
+// words with groups * E <= 4 * kDispThreads).
+constexpr int kDispTableBytes = kDispWarps * CAM_MAX_EXPERTS * 4;
+static_assert(kDispTableBytes >= 2 * 4 * kDispThreads * 4, "the partial column sums must fit");
 
 __device__ __forceinline__ void record_status(CamStatus* st, int code, int who, int detail) {
     if (atomicCAS(&st->code, 0, code) == 0) {
@@ -33,13 +39,163 @@ __device__ __forceinline__ void record_status(CamStatus* st, int code, int who, 
     }
 }
 
+// Inclusive prefix sum of v[0..n) in shared memory, n <= CAM_MAX_EXPERTS, by the whole CTA (s_part: one word per warp).
+// Two values per thread, warp shuffles and one pass over the warps' totals; the serial loops over the experts that this
+// replaces cost every CTA microseconds before its first row (a chain of up to 255 shared-memory reads).
+__device__ __forceinline__ void block_inclusive_scan(int* v, int n, int* s_part) {
+    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5;
+    const int lane = tid & 31;
+    static_assert(CAM_MAX_EXPERTS <= 2 * kDispThreads, "two values per thread must cover all experts");
+    const int i0 = 2 * tid, i1 = i0 + 1;
+    const int a = (i0 < n) ? v[i0] : 0, b = (i1 < n) ? v[i1] : 0;
+    int incl = a + b;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const int o = __shfl_up_sync(0xFFFFFFFFu, incl, s);
+        if (lane >= s) incl += o;
+    }
+    if (lane == 31) s_part[warp] = incl;
+    __syncthreads();
+    int before = 0;
+#pragma unroll
+    for (int w = 0; w < kDispWarps; ++w) before += (w < warp) ? s_part[w] : 0;
+    if (i0 < n) v[i0] = before + incl - b;
+    if (i1 < n) v[i1] = before + incl;
+    __syncthreads();
+}
+
+// A group of one rank exchanges nothing, and a small batch needs not even the grid-wide barrier of the count phase: every
+// CTA counts all ids itself (at most kSmallPairs, 16 KB of shared memory), which gives it the first row of every expert, finds
+// the slots of its own tokens' pairs by scanning the ids, and stores the rows at their places.  At most kSmallTokensPerCta
+// tokens per CTA, one after the other with all threads on a row (int8: four at a time, four warps each); larger batches keep
+// 16 rows in flight per CTA in the general kernel below.  What bounds it is latency: the general kernel spends 24 us on a
+// batch of 16 tokens, 3 of them moving rows (grid barrier and column sums 5, count flag 3, row bases 2, data flag and its
+// system-wide fences 4, the rest one warp quantising a row).  The int8 layer of 16 tokens went from 205 to 166 us with it.
+constexpr int kSmallPairs = 4096, kSmallTokensPerCta = 4;
+static_assert(kSmallPairs * 4 <= kDispTableBytes, "the ids must fit the dynamic shared memory of every quant mode");
+
+__device__ void dispatch_one_rank_small(const DispatchNormalParams& p, uint8_t* dyn_smem, int* s_run, int* s_cum, float* s_red) {
+    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5;
+    const uint32_t lane = lane_id();
+    const int nb = static_cast<int>(gridDim.x), b = static_cast<int>(blockIdx.x);
+    const int E = p.E, K = p.K, npairs = p.T * p.K;
+    const int nscale = CAM_QUANT_IS_FP8(p.quant_mode) ? (p.h >> 7) : (p.quant_mode == CAM_QUANT_INT8_TOKEN) ? 1 : 0;
+    const int row_bytes = (p.quant_mode == CAM_QUANT_NONE) ? p.h * 2 : p.h;
+    const int stage_bytes = (p.quant_mode == CAM_QUANT_NONE) ? 0 : ((p.h + nscale * 4 + 15) & ~15);
+    int* s_ids = reinterpret_cast<int*>(dyn_smem);
+    uint8_t* stage0 = dyn_smem + ((static_cast<size_t>(npairs) * 4 + 15) & ~static_cast<size_t>(15));
+    uint8_t* const base = p.peer_base[p.rank];
+    uint8_t* const rx = base + p.off_recv_x;
+    float* const rs = reinterpret_cast<float*>(base + p.off_recv_scales);
+    int* const tri = reinterpret_cast<int*>(base + p.off_recv_src);
+
+    for (int e = tid; e < E; e += kDispThreads) s_run[e] = 0;
+    __syncthreads();
+    for (int i = tid; i < npairs; i += kDispThreads) {
+        int id = load_expert_id(p.topk_idx, p.idx_is_i64, i);
+        if (id < 0 || id >= E) id = -1;
+        s_ids[i] = id;
+        if (id >= 0) atomicAdd(&s_run[id], 1);
+    }
+    __syncthreads();
+    if (warp == 0) warp_scan_counts(s_run, s_cum, E, lane);
+    __syncthreads();
+    const int total = s_cum[E - 1];
+    const bool fits = total <= p.capacity;
+    if (b == 0) {  // the same bookkeeping as in the general kernel; zero rows are published when they do not fit
+        for (int e = tid; e < E; e += kDispThreads) {
+            const int start = fits ? s_cum[e] - s_run[e] : 0;
+            p.expert_offsets[e] = start;
+            p.recv_count[e] = fits ? s_cum[e] : 0;
+            p.num_recv_per_expert[e] = fits ? static_cast<long long>(s_run[e]) : 0ll;
+            if (p.num_tokens_per_expert_out != nullptr) p.num_tokens_per_expert_out[e] = s_run[e];
+        }
+        if (tid == 0) {
+            p.expert_offsets[E] = fits ? total : 0;
+            p.total_recv[0] = fits ? total : 0;
+            if (!fits) record_status(p.status, CAM_ERR_RECV_OVERFLOW, 0, total);
+            if (p.stats != nullptr) {
+                atomicAdd(&p.stats->rows_routed[0], static_cast<unsigned long long>(total));
+                atomicAdd(&p.stats->calls[0], 1ull);
+            }
+        }
+    }
+    if (p.g1_done != nullptr && b == nb - 1)
+        for (int i = tid; i < p.g1_done_len; i += kDispThreads) p.g1_done[i] = 0u;
+    // Pair k of token t by one warp: its row (or -1), noted for the caller; lanes 0..2 write the origin of a row.
+    auto place = [&](int t, int k) -> int {
+        const int i = t * K + k, id = s_ids[i];
+        int row = -1;
+        if (id >= 0 && fits) {
+            row = s_cum[id] - s_run[id] + warp_slot_of(s_ids, i, lane);
+            if (lane < 3) tri[static_cast<size_t>(row) * 3 + lane] = (lane == 0) ? p.rank : (lane == 1) ? t : k;
+        }
+        if (lane == 0) p.send_row[i] = row;
+        return row;
+    };
+    __shared__ int s_row[4][CAM_MAX_TOPK];
+    if (p.quant_mode == CAM_QUANT_INT8_TOKEN) {
+        const int group = warp >> 2, gw = warp & 3, gt = tid & 127;
+        uint8_t* q = stage0 + static_cast<size_t>(group) * stage_bytes;
+        float* sc = reinterpret_cast<float*>(q + p.h);
+        for (int t = group * nb + b; t < p.T; t += 4 * nb) {  // the first tokens go to different CTAs
+            for (int k = gw; k < K; k += 4) {
+                const int row = place(t, k);
+                if (lane == 0) s_row[group][k] = row;
+            }
+            group_quant_int8_token(p.x + static_cast<size_t>(t) * p.h, p.h, q, sc, nullptr, s_red + group * 4,
+                                   1u + static_cast<uint32_t>(group));
+            for (int k = 0; k < K; ++k) {
+                const int row = s_row[group][k];
+                if (row < 0) continue;
+                uint8_t* dst = rx + static_cast<size_t>(row) * row_bytes;
+                for (int o = gt * 16; o < row_bytes; o += 2048) st_na_v4(dst + o, *reinterpret_cast<const uint4*>(q + o));
+                if (gt == 0) rs[row] = sc[0];
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1u + static_cast<uint32_t>(group)) : "memory");  // staging is free again
+        }
+        return;
+    }
+    const int parts = max(1, kDispWarps / K);
+    const int part_bytes = ((row_bytes + parts - 1) / parts + 511) & ~511;
+    for (int t = b; t < p.T; t += nb) {
+        const __nv_bfloat16* xrow = p.x + static_cast<size_t>(t) * p.h;
+        float* sc = reinterpret_cast<float*>(stage0 + p.h);
+        if (p.quant_mode == CAM_QUANT_FP8_1x128) block_quant_fp8_1x128<false>(xrow, p.h, stage0, sc);
+        else if (p.quant_mode == CAM_QUANT_FP8_1x128_UE8M0) block_quant_fp8_1x128<true>(xrow, p.h, stage0, sc);
+        for (int k = warp; k < K; k += kDispWarps) {
+            const int row = place(t, k);
+            if (lane == 0) s_row[0][k] = row;
+        }
+        __syncthreads();
+        for (int item = warp; item < K * parts; item += kDispWarps) {
+            const int k = item / parts, part = item - k * parts;
+            const int row = s_row[0][k];
+            if (row < 0) continue;
+            uint8_t* dst = rx + static_cast<size_t>(row) * row_bytes;
+            const int b0 = part * part_bytes, b1 = min(row_bytes, b0 + part_bytes);
+            if (p.quant_mode == CAM_QUANT_NONE) {
+                if (b1 > b0) warp_copy_row<false>(dst + b0, reinterpret_cast<const uint8_t*>(xrow) + b0, b1 - b0, lane);
+            } else {
+                for (int o = b0 + static_cast<int>(lane) * 16; o < b1; o += 512)
+                    st_na_v4(dst + o, *reinterpret_cast<const uint4*>(stage0 + o));
+                if (part == 0)
+                    for (int o = static_cast<int>(lane); o < nscale; o += 32) rs[static_cast<size_t>(row) * nscale + o] = sc[o];
+            }
+        }
+        __syncthreads();  // the staged row and the places are overwritten by the next token
+    }
+}
+
 __global__ void __launch_bounds__(kDispThreads, 1)
 dispatch_normal_kernel(const DispatchNormalParams p) {
     extern __shared__ __align__(16) uint8_t dyn_smem[];
     __shared__ int s_hist[CAM_MAX_EXPERTS];     // running per-expert count of this CTA's chunk
     __shared__ int s_aux[CAM_MAX_EXPERTS];      // prefix over earlier CTAs / totals / bases
     __shared__ int s_tot[CAM_MAX_EXPERTS];      // rows per expert summed over all sources
-    __shared__ int s_ids[kDispThreads];
+    __shared__ int s_warp[kDispWarps];
+    __shared__ float s_red[16];
+    int* const s_cum = s_hist;                  // SEND: s_tot summed over experts (inclusive)
     __shared__ int s_rank_ok[CAM_MAX_RANKS];
     __shared__ uint32_t s_abort;
     __shared__ int s_dup_pre[CAM_MAX_RANKS + 1];
@@ -57,31 +213,50 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
     uint8_t* const my_base = p.peer_base[p.rank];
 
     if (tid == 0) s_abort = 0u;
+    // One rank, the whole call in this launch: nothing is exchanged and no flag is raised or waited for.  4096 tokens x 8 of
+    // 7168 (302 MB in and out): 85 us -> 74 us with the parallel column sums and scans, eight loads in flight per lane and
+    // without the flags; the rows themselves move at 6 TB/s.
+    const bool solo = R == 1 && (p.phase_mask & CAM_PHASE_ALL) == CAM_PHASE_ALL && !p.defer_push && p.dbg_drop_flags == 0;
+    if (solo && p.T * K <= kSmallPairs && p.T <= kSmallTokensPerCta * nb) {
+        dispatch_one_rank_small(p, dyn_smem, s_hist, s_tot, s_red);
+        goto done;
+    }
 
     // ------------------------------------------------------------------ phase COUNT
     if (p.phase_mask & CAM_PHASE_COUNT) {
         const int parity = static_cast<int>(ep_count & 1u);
         for (int e = tid; e < E; e += kDispThreads) s_hist[e] = 0;
         __syncthreads();
-        // Slot of every (token, k) pair inside its expert, in scan order, chunk-local first.
+        // Slot of every (token, k) pair inside its expert, in scan order, chunk-local first: match.any gives a pair's
+        // rank among the equal ids of its warp, a warp x expert table of counts the rank of its warp among the 16.
+        int* const tab = reinterpret_cast<int*>(dyn_smem);  // [kDispWarps][E]; the staging rows come later
         for (int sub = 0; sub < npairs; sub += kDispThreads) {
+            for (int o = tid; o < kDispWarps * E; o += kDispThreads) tab[o] = 0;
             const int i = sub + tid;
             int id = -1;
             if (i < npairs) {
                 id = load_expert_id(p.topk_idx, p.idx_is_i64, static_cast<size_t>(t0) * K + i);
                 if (id < 0 || id >= E) id = -1;
             }
-            s_ids[tid] = id;
             __syncthreads();
-            if (id >= 0) {
-                int r = 0;
-                for (int j = 0; j < tid; ++j) r += (s_ids[j] == id) ? 1 : 0;
-                p.slot_in_expert[static_cast<size_t>(t0) * K + i] = s_hist[id] + r;
-            } else if (i < npairs) {
-                p.slot_in_expert[static_cast<size_t>(t0) * K + i] = -1;
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, id);
+            const int before = __popc(same & ((1u << (tid & 31)) - 1u));
+            if (id >= 0 && before == 0) tab[(tid >> 5) * E + id] = __popc(same);
+            __syncthreads();
+            for (int e = tid; e < E; e += kDispThreads) {
+                int run = s_hist[e];
+#pragma unroll
+                for (int w = 0; w < kDispWarps; ++w) {
+                    const int c = tab[w * E + e];
+                    tab[w * E + e] = run;
+                    run += c;
+                }
+                s_hist[e] = run;
             }
             __syncthreads();
-            if (id >= 0) atomicAdd(&s_hist[id], 1);
+            if (i < npairs)
+                p.slot_in_expert[static_cast<size_t>(t0) * K + i] =
+                    (id >= 0) ? tab[(tid >> 5) * E + id] + before : -1;
             __syncthreads();
         }
         for (int e = tid; e < E; e += kDispThreads) p.cta_hist[static_cast<size_t>(b) * E + e] = s_hist[e];
@@ -98,25 +273,60 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
         __threadfence();
         cg::this_grid().sync();
 
-        // Exclusive prefix over earlier CTAs (s_aux) and grand total (s_tot) per expert.
-        for (int e = tid; e < E; e += kDispThreads) {
-            int pre = 0, tot = 0;
-            for (int bb = 0; bb < nb; ++bb) {
-                const int c = __ldcg(&p.cta_hist[static_cast<size_t>(bb) * E + e]);
-                pre += (bb < b) ? c : 0;
-                tot += c;
+        // Exclusive prefix over earlier CTAs (s_aux) and grand total (s_tot) per expert.  The [CTAs, E] table is read by
+        // groups of threads, each group a run of its rows, four experts (one 16-byte load) per thread where E allows, so
+        // that all loads of a thread are in flight together (one thread per expert walking all rows took 10 us and more).
+        {
+            const int vec = ((E & 3) == 0) ? 4 : 1;
+            const int cols = (E + vec - 1) / vec;                      // threads per group
+            const int groups = max(1, min(kDispGroups, kDispThreads / cols));
+            int* const s_pre = reinterpret_cast<int*>(dyn_smem);       // [groups][E], then the totals
+            int* const s_sum = s_pre + groups * E;
+            const int per = (nb + groups - 1) / groups;
+            for (int c0 = 0; c0 < cols; c0 += kDispThreads) {          // more than one pass only for E > 512, vec = 1
+                const int g = (cols <= kDispThreads) ? tid / cols : 0;
+                const int c = c0 + ((cols <= kDispThreads) ? tid - g * cols : tid);
+                if (g < groups && c < cols) {
+                    int pre[4] = {0, 0, 0, 0}, tot[4] = {0, 0, 0, 0};
+                    const int r0 = g * per, r1 = min(nb, r0 + per);
+                    const int* col = p.cta_hist + static_cast<size_t>(c) * vec;
+#pragma unroll 8
+                    for (int bb = r0; bb < r1; ++bb) {
+                        int4 v = make_int4(0, 0, 0, 0);
+                        if (vec == 4) v = __ldcg(reinterpret_cast<const int4*>(col + static_cast<size_t>(bb) * E));
+                        else v.x = __ldcg(col + static_cast<size_t>(bb) * E);
+                        const int m = (bb < b) ? -1 : 0;
+                        pre[0] += v.x & m; pre[1] += v.y & m; pre[2] += v.z & m; pre[3] += v.w & m;
+                        tot[0] += v.x; tot[1] += v.y; tot[2] += v.z; tot[3] += v.w;
+                    }
+                    if (groups == 1) {
+                        for (int u = 0; u < vec; ++u) { s_aux[c * vec + u] = pre[u]; s_tot[c * vec + u] = tot[u]; }
+                    } else {
+                        for (int u = 0; u < vec; ++u) {
+                            s_pre[g * E + c * vec + u] = pre[u];
+                            s_sum[g * E + c * vec + u] = tot[u];
+                        }
+                    }
+                }
             }
-            s_aux[e] = pre;
-            s_tot[e] = tot;
+            __syncthreads();
+            if (groups > 1) {
+                for (int e = tid; e < E; e += kDispThreads) {
+                    int a = 0, t = 0;
+                    for (int g = 0; g < groups; ++g) { a += s_pre[g * E + e]; t += s_sum[g * E + e]; }
+                    s_aux[e] = a;
+                    s_tot[e] = t;
+                }
+                __syncthreads();
+            }
         }
-        __syncthreads();
-        for (int i = tid; i < npairs; i += kDispThreads) {
+        for (int i = tid; !solo && i < npairs; i += kDispThreads) {
             const size_t g = static_cast<size_t>(t0) * K + i;
             const int id = load_expert_id(p.topk_idx, p.idx_is_i64, g);
             if (id >= 0 && id < E) p.slot_in_expert[g] += s_aux[id];
         }
         // Count all-gather: CTA d writes this rank's full count vector into peer d's matrix.
-        for (int d = b; d < R; d += nb) {
+        for (int d = b; !solo && d < R; d += nb) {
             int* dst = reinterpret_cast<int*>(p.peer_base[d] + p.off_count_matrix) +
                        (static_cast<size_t>(parity) * R + p.rank) * E;
             for (int e = tid; e < E; e += kDispThreads) dst[e] = s_tot[e];
@@ -136,7 +346,7 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
     // ------------------------------------------------------------------ phase SEND
     if (p.phase_mask & CAM_PHASE_SEND) {
         const int parity = static_cast<int>(ep_send & 1u);
-        if (tid < R) {
+        if (!solo && tid < R) {
             const uint32_t* f = reinterpret_cast<const uint32_t*>(my_base + p.off_count_flag) + tid;
             const uint64_t t_wait = (b == 0 && p.stats != nullptr) ? globaltimer_ns() : 0ull;
             if (!wait_flag_eq_sys(f, ep_send, p.timeout_ns)) {
@@ -150,30 +360,43 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
 
         const int* cm = reinterpret_cast<const int*>(my_base + p.off_count_matrix) +
                         static_cast<size_t>(parity) * R * E;
-        for (int e = tid; e < E; e += kDispThreads) {
+        // rows for expert e that come from rank s (alone, this rank's totals from the count phase are all there is)
+        auto count_of = [&](int s, int e) { return solo ? s_tot[e] : __ldcg(&cm[static_cast<size_t>(s) * E + e]); };
+        for (int e = tid; !solo && e < E; e += kDispThreads) {
             int tot = 0;
             for (int s = 0; s < R; ++s) tot += __ldcg(&cm[static_cast<size_t>(s) * E + e]);
             s_tot[e] = tot;
         }
         __syncthreads();
+        for (int e = tid; e < E; e += kDispThreads) s_cum[e] = s_tot[e];
+        __syncthreads();
+        block_inclusive_scan(s_cum, E, s_warp);
+        // first row of expert e in its owner's receive buffer
+        auto first_row = [&](int e) {
+            const int lo = e - e % El;
+            return s_cum[e] - s_tot[e] - (lo > 0 ? s_cum[lo - 1] : 0);
+        };
         // Base row, at the owner of expert e, of the block of rows that come from this rank.
         for (int e = tid; e < E; e += kDispThreads) {
-            const int d = e / El, le = e - d * El;
-            int base = 0;
-            for (int l = 0; l < le; ++l) base += s_tot[d * El + l];
-            for (int s = 0; s < p.rank; ++s) base += __ldcg(&cm[static_cast<size_t>(s) * E + e]);
+            int base = first_row(e) + (solo ? s_aux[e] : 0);  // alone, the slots are still counted inside this CTA
+            for (int s = 0; s < p.rank; ++s) base += count_of(s, e);
             s_aux[e] = base;
         }
         for (int d = tid; d < R; d += kDispThreads) {
-            int tot = 0;
-            for (int l = 0; l < El; ++l) tot += s_tot[d * El + l];
+            const int tot = s_cum[d * El + El - 1] - (d > 0 ? s_cum[d * El - 1] : 0);
             s_rank_ok[d] = (tot <= p.capacity) ? 1 : 0;
             if (tot > p.capacity) record_status(p.status, CAM_ERR_RECV_OVERFLOW, d, tot);
-            if (b == 0 && p.stats != nullptr) {
+        }
+        if (b == 0 && p.stats != nullptr) {  // rows this rank routes to every rank: one warp per destination
+            for (int d = tid >> 5; d < R; d += kDispWarps) {
                 int mine = 0;
-                for (int l = 0; l < El; ++l) mine += __ldcg(&cm[static_cast<size_t>(p.rank) * E + d * El + l]);
-                atomicAdd(&p.stats->rows_routed[d], static_cast<unsigned long long>(mine));
-                if (d == 0) atomicAdd(&p.stats->calls[0], 1ull);
+                for (int l = tid & 31; l < El; l += 32) mine += count_of(p.rank, d * El + l);
+#pragma unroll
+                for (int s = 16; s >= 1; s >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, s);
+                if ((tid & 31) == 0) {
+                    atomicAdd(&p.stats->rows_routed[d], static_cast<unsigned long long>(mine));
+                    if (d == 0) atomicAdd(&p.stats->calls[0], 1ull);
+                }
             }
         }
         __syncthreads();
@@ -183,13 +406,11 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
         if (b == 0) {
             const bool fits = s_rank_ok[p.rank] != 0;
             for (int le = tid; le < El; le += kDispThreads) {
-                int start = 0;
-                for (int l = 0; l < le; ++l) start += s_tot[p.rank * El + l];
-                if (!fits) start = 0;
+                const int start = fits ? first_row(p.rank * El + le) : 0;
                 p.expert_offsets[le] = start;
                 int run = start;
                 for (int s = 0; s < R; ++s) {
-                    if (fits) run += __ldcg(&cm[static_cast<size_t>(s) * E + p.rank * El + le]);
+                    if (fits) run += count_of(s, p.rank * El + le);
                     p.recv_count[le * R + s] = run;  // inclusive cumsum, expert major / source minor
                 }
                 p.num_recv_per_expert[le] = fits ? static_cast<long long>(s_tot[p.rank * El + le]) : 0ll;
@@ -344,7 +565,7 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
         // Completion: the last CTA to finish raises this rank's data flag in every peer.
         if (bulk_rows && lane < static_cast<uint32_t>(K)) bulk_wait_group<0>();  // this lane's copies are written
         __syncthreads();
-        if (tid == 0) {
+        if (!solo && tid == 0) {
             __threadfence_system();
             const unsigned int old = atomicAdd(p.done_ctr, 1u);
             if (old == static_cast<unsigned int>(nb - 1)) {
@@ -366,7 +587,7 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
     }
 
     // ------------------------------------------------------------------ phase RECV
-    if (p.phase_mask & CAM_PHASE_RECV) {
+    if ((p.phase_mask & CAM_PHASE_RECV) && !solo) {
         const int parity = static_cast<int>(ep_recv & 1u);
         if (tid < R) {
             const uint32_t* f = reinterpret_cast<const uint32_t*>(my_base + p.off_data_flag) + tid;
@@ -415,6 +636,10 @@ dispatch_normal_kernel(const DispatchNormalParams p) {
     }
 
 done:
+    if ((p.phase_mask & CAM_PHASE_RECV) && p.nums_out != nullptr && b == 0) {  // CTA 0 wrote the counts (this launch or an earlier one)
+        __syncthreads();
+        for (int le = tid; le < p.nums_len; le += kDispThreads) p.nums_out[le] = __ldcg(reinterpret_cast<const long long*>(p.num_recv_per_expert) + le);
+    }
     // the CTA that leaves last advances the epochs of the phases this launch ran
     __syncthreads();
     if (tid == 0 && last_cta_out(p.exit_ctr, static_cast<unsigned int>(nb))) {
@@ -514,10 +739,13 @@ layout_cluster_kernel(const void* topk_idx, int idx_is_i64, int T, int K, int E,
 // ----------------------------------------------------------------------------------------
 // Launchers (C ABI)
 // ----------------------------------------------------------------------------------------
+// Staging rows of the push; the slot table of the count phase and the key counts of the deferred push use the same bytes.
 extern "C" int cam_dispatch_normal_smem_bytes(int h, int quant_mode) {
-    if (quant_mode == CAM_QUANT_NONE) return 0;
+    const int table = cam::kDispTableBytes;  // also holds the ids and four staged rows of a small one-rank call, see below
+    if (quant_mode == CAM_QUANT_NONE) return table;
     const int nscale = CAM_QUANT_IS_FP8(quant_mode) ? h / 128 : 1;
-    return cam::kDispWarps * ((h + nscale * 4 + 15) & ~15);
+    const int staging = cam::kDispWarps * ((h + nscale * 4 + 15) & ~15);
+    return staging > table ? staging : table;
 }
 
 extern "C" int cam_dispatch_normal_max_grid(int device, int h, int quant_mode) {

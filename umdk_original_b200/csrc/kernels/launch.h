@@ -43,6 +43,8 @@ struct DispatchNormalParams {
     int* recv_count;                // [E_local*R] inclusive cumsum (expert major, source minor)
     int* expert_offsets;            // [E_local+1]
     int64_t* num_recv_per_expert;   // [E_local]
+    int64_t* nums_out;              // optional [nums_len]: the caller's copy of num_recv_per_expert (RECV phase)
+    int nums_len;
     int* total_recv;                // [1]
     int* num_tokens_per_expert_out; // [E] optional (may be null)
     unsigned int* done_ctr;         // [1], self-resetting

@@ -693,7 +693,8 @@ static int ensure_deep_workspace(CamBuffer* b) {
 }
 
 static int dispatch_normal_impl(CamBuffer* b, const void* x, const void* topk_idx, int idx_is_i64, int T, int K, int h,
-                                int E, int quant_mode, int phase_mask, bool defer_push, cudaStream_t stream) {
+                                int E, int quant_mode, int phase_mask, bool defer_push, int64_t* nums_out, int nums_len,
+                                cudaStream_t stream) {
     if (check_common(b, T, K, h, E, "dispatch_normal") != 0) return -1;
     CAM_CHECK(T <= b->layout.max_tokens, "dispatch_normal: %d tokens exceed the buffer's max_tokens %d", T, b->layout.max_tokens);
     CAM_CHECK(quant_mode == CAM_QUANT_NONE || quant_mode == CAM_QUANT_INT8_TOKEN || CAM_QUANT_IS_FP8(quant_mode),
@@ -729,6 +730,8 @@ static int dispatch_normal_impl(CamBuffer* b, const void* x, const void* topk_id
     p.recv_count = b->recv_count;
     p.expert_offsets = b->expert_offsets;
     p.num_recv_per_expert = b->num_recv_per_expert;
+    p.nums_out = nums_out;
+    p.nums_len = nums_len;
     p.total_recv = b->total_recv;
     p.num_tokens_per_expert_out = b->num_tokens_per_expert;
     p.done_ctr = b->done_ctr + 0;
@@ -761,7 +764,7 @@ static int dispatch_normal_impl(CamBuffer* b, const void* x, const void* topk_id
 
 extern "C" int cam_dispatch_normal(CamBuffer* b, const void* x, const void* topk_idx, int idx_is_i64, int T, int K,
                                    int h, int E, int quant_mode, int phase_mask, cudaStream_t stream) {
-    return dispatch_normal_impl(b, x, topk_idx, idx_is_i64, T, K, h, E, quant_mode, phase_mask, false, stream);
+    return dispatch_normal_impl(b, x, topk_idx, idx_is_i64, T, K, h, E, quant_mode, phase_mask, false, nullptr, 0, stream);
 }
 
 extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, const int* total_rows, int max_rows,
@@ -1158,8 +1161,8 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
     auto stamp = [&](int i) { if (prof) cudaEventRecord(b->prof_ev[i], stream); };
     stamp(0);
     if (phase_mask & CAM_PHASE_ALL) {
-        if (cam_dispatch_normal(b, x, expert_ids, idx_is_i64, T, K, h, E, CAM_QUANT_INT8_TOKEN, phase_mask & CAM_PHASE_ALL,
-                                stream) != 0)
+        if (dispatch_normal_impl(b, x, expert_ids, idx_is_i64, T, K, h, E, CAM_QUANT_INT8_TOKEN, phase_mask & CAM_PHASE_ALL,
+                                 false, expert_token_nums, El, stream) != 0)
             return -1;
     }
     stamp(1);
@@ -1178,9 +1181,6 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
         if (grouped_gemm_w8a8_impl(b, b->act_q, b->act_s, L.capacity, w2_q, w2_s, b->expert_offsets, El, h, inter, 2,
                                    nullptr, nullptr, nullptr, recv_src, K, stream) != 0)
             return -1;
-        if (expert_token_nums != nullptr)
-            CAM_CUDA(cudaMemcpyAsync(expert_token_nums, b->num_recv_per_expert, sizeof(int64_t) * El,
-                                     cudaMemcpyDeviceToDevice, stream));
     }
     stamp(3);
     if (phase_mask & 8) {
@@ -1210,7 +1210,7 @@ static int fused_moe_deep(CamBuffer* b, const void* x, const void* expert_ids, i
     if (prep_mask) {
         if (ensure_deep_workspace(b) != 0) return -1;
         if (dispatch_normal_impl(b, x, expert_ids, idx_is_i64, T, K, h, E, CAM_QUANT_FP8_1x128_UE8M0, prep_mask,
-                                 own_dispatch, stream) != 0)
+                                 own_dispatch, nullptr, 0, stream) != 0)
             return -1;
     }
     stamp(1);
@@ -1339,8 +1339,9 @@ static int fused_moe_impl(CamBuffer* b, const void* x, const void* expert_ids, i
     auto stamp = [&](int i) { if (prof) cudaEventRecord(b->prof_ev[i], stream); };
     stamp(0);
     if (disp_mask) {
-        if (cam_dispatch_normal(b, x, expert_ids, idx_is_i64, T, K, h, E,
-                                ue8m0 ? CAM_QUANT_FP8_1x128_UE8M0 : CAM_QUANT_FP8_1x128, disp_mask, stream) != 0)
+        if (dispatch_normal_impl(b, x, expert_ids, idx_is_i64, T, K, h, E,
+                                 ue8m0 ? CAM_QUANT_FP8_1x128_UE8M0 : CAM_QUANT_FP8_1x128, disp_mask, false,
+                                 expert_token_nums, El, stream) != 0)
             return -1;
     }
     stamp(1);
@@ -1355,9 +1356,6 @@ static int fused_moe_impl(CamBuffer* b, const void* x, const void* expert_ids, i
         if (grouped_gemm_impl(b, b->act_q, b->act_s, L.capacity, w2_q, w2_s, b->expert_offsets, El, h, inter, 2,
                               nullptr, nullptr, nullptr, recv_src, K, 0, ue8m0, rows_hint, stream) != 0)
             return -1;
-        if (expert_token_nums != nullptr)
-            CAM_CUDA(cudaMemcpyAsync(expert_token_nums, b->num_recv_per_expert, sizeof(int64_t) * El,
-                                     cudaMemcpyDeviceToDevice, stream));
     }
     stamp(3);
     if (phase_mask & 8) {
