@@ -110,7 +110,7 @@ struct CamBuffer {
     // switches read from the environment once, when the buffer is created (UMDK_CAM_GEMM_*, UMDK_CAM_DEEP_FUSE):
     // -1 = not set (the runtime decides), 0 / 1 = forced
     int env_bulk_push = -1, env_pair = -1, env_swap = -1, env_staging2 = -1, env_deep_fuse = -1, env_fuse_lag = -1;
-    std::map<std::tuple<const void*, uint64_t, uint64_t>, std::pair<CUtensorMap, uint64_t>> tmap_cache;  // map, last use
+    std::map<std::tuple<const void*, uint64_t, uint64_t, int>, std::pair<CUtensorMap, uint64_t>> tmap_cache;  // map, last use
     uint64_t tmap_clock = 0;
     std::map<std::tuple<int, int, int, int>, int> ll_grid_cache;  // (h, quant, T, K) -> co-resident grid
 };
@@ -895,10 +895,11 @@ static EncodeTiledFn get_encode_fn() {
 
 constexpr size_t kTmapCacheEntries = 64;
 
-// 2-D byte tensor [rows, inner] with row pitch == inner, boxes of 128 bytes x 128 rows, 128-byte swizzle.
-static int make_tmap(CamBuffer* cache_owner, CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows) {
+// 2-D byte tensor [rows, inner] with row pitch == inner, boxes of 128 bytes x box_rows rows, 128-byte swizzle.
+static int make_tmap(CamBuffer* cache_owner, CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows,
+                     int box_rows = 128) {
     if (cache_owner != nullptr) {
-        auto it = cache_owner->tmap_cache.find(std::make_tuple(base, inner, rows));
+        auto it = cache_owner->tmap_cache.find(std::make_tuple(base, inner, rows, box_rows));
         if (it != cache_owner->tmap_cache.end()) {
             *out = it->second.first;
             it->second.second = ++cache_owner->tmap_clock;
@@ -913,7 +914,7 @@ static int make_tmap(CamBuffer* cache_owner, CUtensorMap* out, const void* base,
     CAM_CHECK(rows >= 1, "tensor map needs at least one row");
     cuuint64_t dims[2] = {inner, rows};
     cuuint64_t strides[1] = {inner};
-    cuuint32_t box[2] = {128, 128};
+    cuuint32_t box[2] = {128, static_cast<cuuint32_t>(box_rows)};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -927,13 +928,10 @@ static int make_tmap(CamBuffer* cache_owner, CUtensorMap* out, const void* base,
                 if (c->second.second < oldest->second.second) oldest = c;
             cache_owner->tmap_cache.erase(oldest);
         }
-        cache_owner->tmap_cache[std::make_tuple(base, inner, rows)] = std::make_pair(*out, ++cache_owner->tmap_clock);
+        cache_owner->tmap_cache[std::make_tuple(base, inner, rows, box_rows)] = std::make_pair(*out, ++cache_owner->tmap_clock);
     }
     return 0;
 }
-
-// Mean rows per expert below which the block-scaled GEMM runs with its operands exchanged (0 = never by default).
-constexpr int kSwapRowsPerExpert = 0;
 
 static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scales, int a_rows, const void* w_q,
                              const float* w_scales, const int* expert_offsets, int num_experts, int n_dim, int k_dim,
@@ -959,9 +957,6 @@ static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scale
     } else {
         CAM_CUDA(cudaGetDevice(&device));
     }
-    CUtensorMap ta, tb;
-    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows)) != 0) return -1;
-    if (make_tmap(b, &tb, w_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(num_experts) * n_dim) != 0) return -1;
     cam::GroupedGemmParams p{};
     p.expert_offsets = expert_offsets;
     p.num_experts = num_experts;
@@ -1022,19 +1017,28 @@ static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scale
     // UMDK_CAM_GEMM_PAIR=0/1 forces the choice.
     bool pair = ue8m0 && rows_per_expert_hint >= 384;
     if (sw_pair >= 0) pair = ue8m0 && sw_pair == 1;
-    // Small experts (a tile of rows or less each) take the kernel with the operands exchanged, whose tensor-core
-    // time follows the rows actually present instead of whole 128-row tiles; UMDK_CAM_GEMM_SWAP=0/1 forces the choice.
-    bool swap = ue8m0 && !pair && rows_per_expert_hint < kSwapRowsPerExpert;
-    if (sw_swap >= 0) swap = ue8m0 && !pair && sw_swap == 1;
+    // Below that, the kernel with the operands exchanged (the rows as N operand, grouped_gemm_rows_n.cuh): every weight byte
+    // crosses to the SMs once and the tensor time follows the rows present.  Layers of 7168 x 2048 experts in a steady loop,
+    // this kernel against the CTA pairs with 256-row tiles: 4 rows per expert (256 experts) 1.76 / 3.03 ms, 128 rows 2.65 /
+    // 3.45 ms, 256 rows (64 experts) 1.13 / 1.23 ms, 750 rows (32) 1.27 / 1.25 ms, 4096 rows of 2048 x 1024 0.62 / 0.56 ms;
+    // 512 rows go either way (1.82 / 1.95 ms; 4096 x 1536 experts 1.77 / 1.74 ms).  UMDK_CAM_GEMM_SWAP=0 forces the one-CTA
+    // kernel instead, which is also the form without bulk copies.
+    const bool rows_n = ue8m0 && !pair && p.bulk_push != 0 && sw_swap != 0;
     // The combine-send epilogue of the block-scaled kernels overlaps converting a half tile with the copies of the previous
     // one (two staging buffers, paid for with pipeline stages); UMDK_CAM_GEMM_STAGING2=0 keeps the one-buffer form.
     // On by default in the CTA-pair kernel only: the one-CTA kernel, used for small experts, lives on streaming weights
     // and loses more from its fourth pipeline stage than the epilogue gains (measured on one GPU, 256 experts).
     bool two_staging = mode == 2 && p.bulk_push != 0 && pair;
     if (sw_stg2 >= 0) two_staging = mode == 2 && p.bulk_push != 0 && sw_stg2 == 1;
-    const int rc = !ue8m0 ? cam_launch_grouped_gemm_fp8(&p, &ta, &tb, sms, stream)
-                   : pair ? cam_launch_grouped_gemm_mxfp8_pair(&p, &ta, &tb, sms, two_staging ? 1 : 0, stream)
-                          : cam_launch_grouped_gemm_mxfp8(&p, &ta, &tb, sms, swap ? 1 : 0, two_staging ? 1 : 0, stream);
+    CUtensorMap ta, tb;
+    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows),
+                  rows_n ? cam_grouped_gemm_rows_n_box() : 128) != 0)
+        return -1;
+    if (make_tmap(b, &tb, w_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(num_experts) * n_dim) != 0) return -1;
+    const int rc = !ue8m0   ? cam_launch_grouped_gemm_fp8(&p, &ta, &tb, sms, stream)
+                   : rows_n ? cam_launch_grouped_gemm_mxfp8_rows_n(&p, &ta, &tb, sms, stream)
+                   : pair   ? cam_launch_grouped_gemm_mxfp8_pair(&p, &ta, &tb, sms, two_staging ? 1 : 0, stream)
+                            : cam_launch_grouped_gemm_mxfp8(&p, &ta, &tb, sms, two_staging ? 1 : 0, stream);
     CAM_CHECK(rc == 0, "grouped_gemm launch failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
     if (b != nullptr) ++b->launches;
     return 0;
@@ -1084,7 +1088,8 @@ static int grouped_gemm_w8a8_impl(CamBuffer* b, const void* a_q, const float* a_
         CAM_CUDA(cudaGetDevice(&device));
     }
     CUtensorMap ta, tb;
-    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows)) != 0) return -1;
+    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows), cam_grouped_gemm_rows_n_box()) != 0)
+        return -1;
     if (make_tmap(b, &tb, w_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(num_experts) * n_dim) != 0) return -1;
     cam::GroupedGemmParams p{};
     p.expert_offsets = expert_offsets;
@@ -1128,7 +1133,7 @@ static int grouped_gemm_w8a8_impl(CamBuffer* b, const void* a_q, const float* a_
     }
     int sms = 0;
     CAM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int rc = cam_launch_grouped_gemm_w8a8(&p, &ta, &tb, sms, stream);
+    const int rc = cam_launch_grouped_gemm_w8a8_rows_n(&p, &ta, &tb, sms, stream);
     CAM_CHECK(rc == 0, "grouped_gemm_w8a8 launch failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
     if (b != nullptr) ++b->launches;
     return 0;
