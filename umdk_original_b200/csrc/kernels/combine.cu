@@ -291,6 +291,40 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
             const int o_end = min(row_bytes, o_begin + per * 512);
             const uint32_t valid = load_pairs(t);
             uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(t) * row_bytes;
+            if (p.K <= 8) {
+                // The loads of the next 512 bytes of all rows are in flight while these are added up: with one batch at a
+                // time a warp has nothing outstanding between its last load and the store (4096 tokens x 8 rows of 14 KB:
+                // 102.6 -> 94.7 us, 5.6 TB/s).
+                auto load8 = [&](uint4 (&v)[8], int o) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        v[k] = ((valid >> k) & 1u) ? ld_cg_v4(reinterpret_cast<const uint8_t*>(s_row[warp][k] & ~1ull) + o)
+                                                   : make_uint4(0, 0, 0, 0);
+                };
+                auto add8 = [&](const uint4 (&v)[8], int o) {
+                    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if ((valid >> k) & 1u) fma_bf16x8(acc, v[k], s_w[warp][k]);
+                    uint4 r;
+                    r.x = pack_bf16x2(acc[0], acc[1]);
+                    r.y = pack_bf16x2(acc[2], acc[3]);
+                    r.z = pack_bf16x2(acc[4], acc[5]);
+                    r.w = pack_bf16x2(acc[6], acc[7]);
+                    st_na_v4(orow + o, r);
+                };
+                uint4 va[8], vb[8];
+                int o = o_begin + static_cast<int>(lane) * 16;
+                if (o < o_end) load8(va, o);
+                for (; o < o_end; o += 1024) {
+                    if (o + 512 < o_end) load8(vb, o + 512);
+                    add8(va, o);
+                    if (o + 1024 < o_end) load8(va, o + 1024);
+                    if (o + 512 < o_end) add8(vb, o + 512);
+                }
+                __syncwarp();
+                continue;
+            }
             for (int o = o_begin + static_cast<int>(lane) * 16; o < o_end; o += 512) {
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 for (int k0 = 0; k0 < p.K; k0 += 8) {
