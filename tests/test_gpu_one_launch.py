@@ -141,3 +141,29 @@ def test_prefill_dispatch_formats_in_one_launch(t, h, e, k, quant):
     stats = buf.stats()
     assert stats["dispatch_calls"] == 1 and stats["rows_routed_to_peer"] == [n]
     buf.destroy()
+
+
+@pytest.mark.parametrize("t", [9, 700])  # the short form, and the general kernel of a rank alone
+def test_receive_overflow_in_one_launch(t):
+    e, k, h = 4, 2, 128
+    idx, w, g = _routing(t, e, k, seed=t, skip=0)
+    cap = t * k - 1
+    buf = u.Buffer(None, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, capacity=cap, timeout_ms=2000.0), device=DEV,
+                   rank=0, num_ranks=1)
+    region = buf.native.recv_x(cap, h, 0)
+    region.fill_(7.0)
+    canary = region.clone()
+    x = torch.randn(t, h, generator=g).to(torch.bfloat16)
+    per_e = ops.moe_dispatch_prefill_quant(x.to(DEV), idx.to(DEV), w.to(DEV), cap, buf.name, 0, 1, 0)[3]
+    with pytest.raises(u.RecvOverflow) as ei:
+        buf.check()
+    assert ei.value.who == 0 and ei.value.detail == t * k
+    assert int(buf.native.total_recv().item()) == 0 and int(per_e.sum().item()) == 0
+    assert int(buf.native.expert_offsets(e + 1).abs().sum().item()) == 0
+    assert bool((buf.native.send_row(t * k) == -1).all()) and torch.equal(region, canary)
+    buf.reset()
+    idx[1:] = -1  # after the reset a call that fits goes through
+    rx = ops.moe_dispatch_prefill_quant(x.to(DEV), idx.to(DEV), w.to(DEV), 0, buf.name, 0, 1, 0)[0]
+    buf.check()
+    assert torch.equal(rx.cpu(), x[:1].expand(k, h))
+    buf.destroy()
