@@ -466,21 +466,26 @@ extern "C" int cam_dispatch_ll_smem_bytes(int h, int quant_mode, int T, int K, i
     return ((T * K * 8 + 15) & ~15) + (per_group > shared_row ? per_group : shared_row);
 }
 
+// One record of the kernel's shared-memory limit for the occupancy query and the launch: the limit only ever grows, so a
+// query for a small shape does not lower it under a launch of a larger shape seen before.
+static cam::SmemLimitCache g_ll_smem_limit;
+
 extern "C" int cam_dispatch_ll_max_grid(int device, int h, int quant_mode, int T, int K, int E) {
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -1;
     const int smem = cam_dispatch_ll_smem_bytes(h, quant_mode, T, K, E);
-    cudaFuncSetAttribute(cam::dispatch_ll_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cam::dispatch_ll_kernel, cam::kLLThreads, smem) !=
-        cudaSuccess)
+    if (g_ll_smem_limit.ensure(cam::dispatch_ll_kernel, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cam::dispatch_ll_kernel, cam::kLLThreads, smem) !=
+            cudaSuccess) {
+        cudaGetLastError();  // the refusal is this call's, not the next launch's
         return -1;
+    }
     return sms * per_sm;
 }
 
 extern "C" int cam_launch_dispatch_ll(const cam::DispatchLLParams* p, int grid, cudaStream_t stream) {
     const int smem = cam_dispatch_ll_smem_bytes(p->h, p->quant_mode, p->T, p->K, p->E);
-    static cam::SmemLimitCache limit;
-    cudaError_t e = limit.ensure(cam::dispatch_ll_kernel, smem);
+    cudaError_t e = g_ll_smem_limit.ensure(cam::dispatch_ll_kernel, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
     void* args[] = {const_cast<cam::DispatchLLParams*>(p)};
     return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(cam::dispatch_ll_kernel), dim3(grid),

@@ -748,17 +748,6 @@ extern "C" int cam_dispatch_normal_smem_bytes(int h, int quant_mode) {
     return staging > table ? staging : table;
 }
 
-extern "C" int cam_dispatch_normal_max_grid(int device, int h, int quant_mode) {
-    int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -1;
-    const int smem = cam_dispatch_normal_smem_bytes(h, quant_mode);
-    cudaFuncSetAttribute(cam::dispatch_normal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cam::dispatch_normal_kernel, cam::kDispThreads,
-                                                      smem) != cudaSuccess)
-        return -1;
-    return sms * (per_sm > 0 ? 1 : 0);
-}
-
 extern "C" int cam_launch_dispatch_normal(const cam::DispatchNormalParams* p, int grid, cudaStream_t stream) {
     const int smem = cam_dispatch_normal_smem_bytes(p->h, p->quant_mode);
     static cam::SmemLimitCache limit;

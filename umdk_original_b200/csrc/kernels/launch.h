@@ -6,6 +6,10 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
+#include <mutex>
+
 #include "../common/cam_types.h"
 
 namespace cam {
@@ -219,18 +223,25 @@ struct TpExchangeParams {
 };
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) costs microseconds per call; the launchers go
-// through this helper, which remembers per device what it has already set for one kernel.
+// through this helper, which remembers per device what it has already set for one kernel.  The limit
+// only grows (under a lock: two threads must not set it in the wrong order), so everything that sets
+// it for a kernel shares one of these.  A refused size leaves no error behind for the next launch.
 struct SmemLimitCache {
-    int set[64] = {0};
+    std::atomic<int> set[64] = {};
+    std::mutex lock;
     template <class Kernel>
     cudaError_t ensure(Kernel k, int bytes) {
+        if (bytes <= 0) return cudaSuccess;
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64 && set[dev] >= bytes && bytes > 0) return cudaSuccess;
-        if (bytes <= 0) return cudaSuccess;
+        const bool known = dev >= 0 && dev < 64;
+        if (known && set[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+        std::lock_guard<std::mutex> guard(lock);
+        if (known && set[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e == cudaSuccess && dev >= 0 && dev < 64) set[dev] = bytes;
+        if (e != cudaSuccess) cudaGetLastError();
+        else if (known) set[dev].store(bytes, std::memory_order_release);
         return e;
     }
 };
@@ -251,7 +262,6 @@ inline int sm_count_of_current_device() {
 
 extern "C" {
 int cam_dispatch_normal_smem_bytes(int h, int quant_mode);
-int cam_dispatch_normal_max_grid(int device, int h, int quant_mode);
 int cam_launch_dispatch_normal(const cam::DispatchNormalParams* p, int grid, cudaStream_t stream);
 int cam_launch_layout(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R,
                       int* num_tokens_per_rank, int* num_tokens_per_expert, uint8_t* is_token_in_rank,
