@@ -15,7 +15,7 @@ DEV = torch.device("cuda", 0)
 @pytest.fixture(params=["single", "pair", "swap"])
 def gemm_variant(request, monkeypatch):
     """Runs a block-scaled GEMM test on the one-CTA kernel, on the CTA-pair (cta_group::2) kernel and on the
-    one-CTA kernel with its operands exchanged (weights as the M operand, for small experts)."""
+    CTA-pair kernel with its operands exchanged (weights as the M operand, rows as the N operand)."""
     monkeypatch.setenv("UMDK_CAM_GEMM_PAIR", "1" if request.param == "pair" else "0")
     monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", "1" if request.param == "swap" else "0")
     return request.param

@@ -58,15 +58,22 @@ def _sample_rows(counts, per_expert, seed):
     return picks
 
 
-@pytest.fixture(params=["fp32_scales", "mx_single", "mx_pair"])
+@pytest.fixture(params=["fp32_scales", "mx_single", "mx_pair", "mx_rows_n"])
 def big_variant(request, monkeypatch):
     monkeypatch.setenv("UMDK_CAM_GEMM_PAIR", "1" if request.param == "mx_pair" else "0")
-    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", "0")
+    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", "1" if request.param == "mx_rows_n" else "0")
+    return request.param
+
+
+@pytest.fixture(params=["single", "rows_n"])
+def int8_variant(request, monkeypatch):
+    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", "1" if request.param == "rows_n" else "0")
     return request.param
 
 
 def test_grouped_gemm_plain_many_tiles_per_cta(big_variant):
-    """24 ragged experts x N = 2048 x K = 7168: about 700 (one-CTA kernels) / 400 (CTA pairs) output tiles."""
+    """24 ragged experts x N = 2048 x K = 7168: about 700 (one-CTA kernels) / 400 (CTA pairs) / 200 (rows as N operand, 74 CTA
+    pairs, tiles of up to 128 and of more rows in turn) output tiles."""
     ue8m0 = big_variant != "fp32_scales"
     counts = _ragged_counts(24, 700, seed=5)
     n, k = 2048, 7168
@@ -108,7 +115,7 @@ def test_grouped_gemm_swiglu_requant_many_tiles_per_cta(big_variant):
         assert ref.is_power_of_two(s[: sum(counts)].cpu())
 
 
-def test_grouped_gemm_w8a8_many_tiles_per_cta():
+def test_grouped_gemm_w8a8_many_tiles_per_cta(int8_variant):
     """int8 x int8 -> int32 at K = 7168: the integer sums are exact, so sampled rows must agree to bf16 rounding."""
     counts = _ragged_counts(16, 600, seed=13)
     n, k = 2048, 7168

@@ -1,6 +1,8 @@
 """GPU tests of the grouped GEMM whose rows are the tensor core's N operand (CTA pairs), in its three arithmetics, against the
-CPU oracle: expert sizes round the steps of its tiles, weight blocks that do not fill the last tile, short reductions."""
+CPU oracle: expert sizes round the steps of its tiles, weight blocks that do not fill the last tile, short reductions.  The int8
+tests run the one-CTA kernel as well, and the last test compares the two on either side of the lines between them."""
 import pytest
+import test_gpu_gemm_fused as layer_tests
 import torch
 
 import umdk_original_b200 as u  # noqa: F401
@@ -19,6 +21,7 @@ SHAPES = [(128, 128), (384, 512), (512, 640), (1280, 1152)]
 @pytest.fixture(autouse=True)
 def _form(monkeypatch):
     monkeypatch.setenv("UMDK_CAM_GEMM_PAIR", "0")
+    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", "1")
 
 
 def _fp8_problem(counts, n, k, po2):
@@ -61,9 +64,11 @@ def test_swiglu_requant(counts, inter, k, po2):
     assert ((ratio - 1).abs() < 1e-4).float().mean() > (0.98 if po2 else 0.999)
 
 
+@pytest.mark.parametrize("swap", ["0", "1"])
 @pytest.mark.parametrize("n,k", SHAPES)
 @pytest.mark.parametrize("counts", COUNTS)
-def test_int8(counts, n, k):
+def test_int8(counts, n, k, swap, monkeypatch):
+    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", swap)
     g = torch.Generator().manual_seed(sum(counts) + n + k)
     a = torch.randint(-127, 128, (sum(counts), k), generator=g).to(torch.int8)
     w = torch.randint(-127, 128, (len(counts), n, k), generator=g).to(torch.int8)
@@ -74,3 +79,32 @@ def test_int8(counts, n, k):
     want = ops.grouped_gemm_w8a8(*p).float()
     # exact integers, two fp32 products, one bf16 rounding: at most one bf16 step
     assert ((got - want).abs() <= 2.0 ** -7 * want.abs()).all()
+
+
+@pytest.mark.parametrize("swap", ["0", "1"])
+@pytest.mark.parametrize("world", [1, 2])
+def test_int8_layer(world, swap, monkeypatch):
+    monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", swap)
+    layer_tests.test_fused_moe_w8a8_reference_layout(world)
+
+
+@pytest.mark.parametrize("e,n,k,rows", [
+    (30, 4096, 1536, 3), (31, 4096, 1536, 3),     # 189 and 195 MB of weights
+    (31, 3968, 1536, 65), (32, 4096, 1536, 113),  # 6.1 M weights per expert and the full 128-row tiles; past them
+    (47, 1024, 6144, 2), (48, 1024, 6144, 2),     # 94 and 96 tiles
+    (40, 1536, 3840, 2)])                         # 5.9 M weights per expert
+def test_the_choice_changes_no_byte(e, n, k, rows, monkeypatch):
+    # int8 sums are exact and the scales are applied in one order, so both forms and the default give the same bytes
+    g = torch.Generator(device=DEV).manual_seed(e + n)
+    a = torch.randint(-127, 128, (e * rows, k), device=DEV, generator=g).to(torch.int8)
+    w = torch.randint(-127, 128, (e, n, k), device=DEV, generator=g, dtype=torch.int8)
+    a_s, w_s = torch.rand(e * rows, device=DEV, generator=g) + 0.01, torch.rand(e, n, device=DEV, generator=g) + 0.01
+    off = torch.arange(0, e * rows + 1, rows, dtype=torch.int32, device=DEV)
+    got = {}
+    for swap in ("", "0", "1"):
+        monkeypatch.setenv("UMDK_CAM_GEMM_SWAP", swap)
+        got[swap] = ops.grouped_gemm_w8a8(a, a_s, w, w_s, off).view(torch.int16)
+    assert torch.equal(got[""], got["0"]) and torch.equal(got[""], got["1"])
+    last = slice((e - 1) * rows, e * rows)
+    want = (a[last].double() @ w[e - 1].double().t()).float() * a_s[last, None] * w_s[e - 1]
+    assert torch.equal(got[""][last], want.to(torch.bfloat16).view(torch.int16))

@@ -31,8 +31,9 @@
 // Every mbarrier wait is bounded; a role that gives up sets a shared abort word that releases
 // the others, a status word is recorded and the CTA frees its TMEM and returns.
 //
-// grouped_gemm_rows_n.cuh exchanges the operands and is the default for experts that do not fill the 256-row tiles of
-// grouped_gemm_mx2.cu; this kernel serves UMDK_CAM_GEMM_SWAP=0 and the form without bulk copies (UMDK_CAM_GEMM_BULK_PUSH=0).
+// grouped_gemm_rows_n.cuh exchanges the operands and serves experts that do not fill the 256-row tiles of grouped_gemm_mx2.cu
+// when there are enough large weights; this kernel serves the rest (cam_grouped_gemm_rows_n_pays in cam_runtime.cpp has the line and the times on
+// both sides of it) and the form without bulk copies (UMDK_CAM_GEMM_BULK_PUSH=0).
 #include "gemm_common.cuh"
 
 namespace cam {

@@ -10,6 +10,7 @@
 // Measured with 7168 x 2048 experts on one GPU: 256 experts x 128 rows, first GEMM 1.44 -> 1.27 ms (5.9 TB/s of weights),
 // second 0.78 -> 0.70 ms; the layer in a steady loop, where the 1 kW limit holds the clock down and padded tensor work costs
 // twice, 3.15 -> 2.62 ms; 4 rows per expert 2.15 -> 1.78 ms (6.9 TB/s).  A bare TMA read stream reaches 6.9 - 7.1 TB/s.
+// Short reductions and few tiles are dearer here than on one CTA: cam_grouped_gemm_rows_n_pays in cam_runtime.cpp keeps those away.
 //
 // One tile: 512 weight rows (each CTA two blocks of 128: the gate and the up block of the same 128 features for the SwiGLU
 // GEMM, two neighbouring blocks of output features otherwise) x N rows, K in steps of 128.  Tensor memory of each CTA

@@ -283,6 +283,8 @@ int cam_launch_grouped_gemm_mxfp8_rows_n(const cam::GroupedGemmParams* p, const 
                                          const CUtensorMap* tmap_b, int grid, cudaStream_t stream);
 int cam_launch_grouped_gemm_w8a8_rows_n(const cam::GroupedGemmParams* p, const CUtensorMap* tmap_a,
                                         const CUtensorMap* tmap_b, int grid, cudaStream_t stream);
+int cam_launch_grouped_gemm_w8a8(const cam::GroupedGemmParams* p, const CUtensorMap* tmap_a,
+                                 const CUtensorMap* tmap_b, int grid, cudaStream_t stream);
 int cam_launch_grouped_gemm_mxfp8_pair(const cam::GroupedGemmParams* p, const CUtensorMap* tmap_a,
                                        const CUtensorMap* tmap_b, int grid, int two_staging, cudaStream_t stream);
 int cam_grouped_gemm_mx_pair_smem_bytes(void);

@@ -2,8 +2,8 @@
 // with one scale per output channel, int32 accumulation (fused_deep_moe/gemm/kernel/grouped_matmul_slice_m_per_token_dequant_
 // swiglu_quant_multistage_workspace.h:558-632 on the cube cores, dequantisation in
 // epilogue/block/block_epilogue_per_token_dequant_swiglu.h:236-272 and block_epilogue_per_token_dequant.hpp:664-684 on the
-// vector cores).  The two GEMMs are the int8 form of grouped_gemm_rows_n.cuh (a_scales [rows], one per token; b_scales [E, N],
-// one per output channel); its mode 1 leaves fp32 activations and the maximum of |.| of every row, from which the pass below
+// vector cores).  The two GEMMs are grouped_gemm_i8.cu or the int8 form of grouped_gemm_rows_n.cuh (a_scales [rows], one per token;
+// b_scales [E, N], one per output channel); their mode 1 leaves fp32 activations and the maximum of |.| of every row, from which the pass below
 // derives the per-token scale of the second GEMM's activations (the reference's BlockQuant pass, ...workspace.h:161-277).
 #include "gemm_common.cuh"
 

@@ -207,6 +207,13 @@ extern "C" int cam_layout_compute_tp(CamLayout* L, int R, int E, int max_tokens,
     return 0;
 }
 
+// Switches: a Buffer reads UMDK_CAM_GEMM_* once when it is created; the stand-alone ops (no Buffer) read the environment
+// per call.  -1 = not set.
+static int env_now(const char* name) {
+    const char* v = getenv(name);
+    return (v == nullptr || v[0] == '\0') ? -1 : atoi(v);
+}
+
 extern "C" CamBuffer* cam_buffer_create(int device, int rank, int num_ranks, const CamLayout* layout) {
     auto bad = [](const char* what, cudaError_t e) -> CamBuffer* {
         fail("%s failed: %s", what, cudaGetErrorString(e));
@@ -223,16 +230,12 @@ extern "C" CamBuffer* cam_buffer_create(int device, int rank, int num_ranks, con
     b->rank = rank;
     b->num_ranks = num_ranks;
     b->layout = *layout;
-    auto env_switch = [](const char* name) {
-        const char* v = getenv(name);
-        return (v == nullptr || v[0] == '\0') ? -1 : atoi(v);
-    };
-    b->env_bulk_push = env_switch("UMDK_CAM_GEMM_BULK_PUSH");
-    b->env_pair = env_switch("UMDK_CAM_GEMM_PAIR");
-    b->env_swap = env_switch("UMDK_CAM_GEMM_SWAP");
-    b->env_staging2 = env_switch("UMDK_CAM_GEMM_STAGING2");
-    b->env_deep_fuse = env_switch("UMDK_CAM_DEEP_FUSE");
-    b->env_fuse_lag = env_switch("UMDK_CAM_FUSE_LAG");
+    b->env_bulk_push = env_now("UMDK_CAM_GEMM_BULK_PUSH");
+    b->env_pair = env_now("UMDK_CAM_GEMM_PAIR");
+    b->env_swap = env_now("UMDK_CAM_GEMM_SWAP");
+    b->env_staging2 = env_now("UMDK_CAM_GEMM_STAGING2");
+    b->env_deep_fuse = env_now("UMDK_CAM_DEEP_FUSE");
+    b->env_fuse_lag = env_now("UMDK_CAM_FUSE_LAG");
     const int E = layout->num_experts, R = num_ranks;
     if ((e = cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) {
         delete b;
@@ -933,6 +936,25 @@ static int make_tmap(CamBuffer* cache_owner, CUtensorMap* out, const void* base,
     return 0;
 }
 
+// Rows-as-N kernel (grouped_gemm_rows_n.cuh) or one-CTA kernel (grouped_gemm_mx.cu, grouped_gemm_i8.cu).  The first moves every
+// weight byte to the SMs once and pads rows to 16 or 32, but a pair of CTAs takes 512 weight rows at a time, walks the
+// experts tile by tile and drains one set of accumulators: short reductions and few tiles are dearer on it.  Times against
+// the one-CTA kernel in a steady loop, 32 to 256 experts, 1 to 380 rows each (one B200, weights N x K per expert):
+//   outputs (modes 0, 2)  2048 x 1024 1.05 - 1.57, 4096 x 1024 0.83 - 1.24, 2048 x 2048 0.81 - 1.16,
+//                         4096 x 1536 0.74 - 1.10, 7168 x 2048 0.70 - 1.03
+//   SwiGLU (mode 1)       4096 x 1024 0.99 - 1.33, 2048 x 2048 0.90 - 1.18, 3072 x 2048 0.81 - 1.12,
+//                         2048 x 4096 0.73 - 1.10, 4096 x 7168 0.66 - 1.04
+// The weights of a call have to be more than the L2 keeps, and the tiles more than the 74 pairs: 134 MB of 8.4 M weights each
+// (16 experts) 0.87 - 1.11, 201 MB of 6.3 M 0.87 - 1.10; 64 tiles of 7168 x 4096 SwiGLU (8 experts) 0.77 - 1.17, 128 tiles (16)
+// 0.71 - 1.04.  Between 64 and 112 rows the one-CTA kernel's 128-row tiles are nearly full and it is 3 to 10 % ahead up to
+// 16 M weights per expert (4096 x 7168: level).
+extern "C" int cam_grouped_gemm_rows_n_pays(int num_experts, int rows_per_expert, int n_dim, int k_dim, int mode) {
+    const int64_t weights = static_cast<int64_t>(n_dim) * k_dim;
+    if (weights < (mode == 1 ? 8000000 : 6000000) || num_experts * weights < 190000000) return 0;
+    if (static_cast<int64_t>(num_experts) * ((n_dim + 511) / 512) < 96) return 0;
+    return rows_per_expert <= 64 || rows_per_expert > 112 || weights >= 16000000;
+}
+
 static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scales, int a_rows, const void* w_q,
                              const float* w_scales, const int* expert_offsets, int num_experts, int n_dim, int k_dim,
                              int mode, void* out_bf16, void* act_q, float* act_s, const int* row_src, int topk,
@@ -1000,12 +1022,6 @@ static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scale
     p.topk = topk;
     int sms = 0;
     CAM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    // Switches: a Buffer reads UMDK_CAM_GEMM_* once when it is created; the stand-alone ops (no Buffer) read the
-    // environment per call.  -1 = not set.
-    auto env_now = [](const char* name) {
-        const char* v = getenv(name);
-        return (v == nullptr || v[0] == '\0') ? -1 : atoi(v);
-    };
     const int sw_bulk = b ? b->env_bulk_push : env_now("UMDK_CAM_GEMM_BULK_PUSH");
     const int sw_pair = b ? b->env_pair : env_now("UMDK_CAM_GEMM_PAIR");
     const int sw_swap = b ? b->env_swap : env_now("UMDK_CAM_GEMM_SWAP");
@@ -1013,17 +1029,18 @@ static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scale
     // rows leave the GEMM2 epilogue as 256-byte bulk copies (measured a few percent ahead of vector stores at 2 and 4
     // GPUs); UMDK_CAM_GEMM_BULK_PUSH=0 selects the vector-store form
     p.bulk_push = sw_bulk < 0 ? 1 : (sw_bulk == 1);
-    // CTA pairs (256-row tiles, B tile shared inside the cluster) pay off once experts fill such tiles;
+    // CTA pairs (256-row tiles, B tile shared inside the cluster) pay off once experts fill such tiles: 384, 512 and 768 rows
+    // take 0.92, 1.02 and 1.01 of the one-CTA kernel's time with 2048 x 4096 SwiGLU experts (32 and 64 of them, a steady loop).
+    // With large weights the rows-as-N kernel keeps up with them beyond this line: 7168 x 4096 SwiGLU 0.70 - 0.89 of the pairs'
+    // time at 384 rows, 0.90 - 0.97 at 512, 0.91 - 0.96 at 768 and more; 2048 x 4096 0.93 - 0.98, 1.05 - 1.12, 1.04 - 1.12.
     // UMDK_CAM_GEMM_PAIR=0/1 forces the choice.
     bool pair = ue8m0 && rows_per_expert_hint >= 384;
     if (sw_pair >= 0) pair = ue8m0 && sw_pair == 1;
-    // Below that, the kernel with the operands exchanged (the rows as N operand, grouped_gemm_rows_n.cuh): every weight byte
-    // crosses to the SMs once and the tensor time follows the rows present.  Layers of 7168 x 2048 experts in a steady loop,
-    // this kernel against the CTA pairs with 256-row tiles: 4 rows per expert (256 experts) 1.76 / 3.03 ms, 128 rows 2.65 /
-    // 3.45 ms, 256 rows (64 experts) 1.13 / 1.23 ms, 750 rows (32) 1.27 / 1.25 ms, 4096 rows of 2048 x 1024 0.62 / 0.56 ms;
-    // 512 rows go either way (1.82 / 1.95 ms; 4096 x 1536 experts 1.77 / 1.74 ms).  UMDK_CAM_GEMM_SWAP=0 forces the one-CTA
-    // kernel instead, which is also the form without bulk copies.
-    const bool rows_n = ue8m0 && !pair && p.bulk_push != 0 && sw_swap != 0;
+    // Below that, the rows-as-N kernel or the one-CTA kernel, which is also the form without bulk copies;
+    // UMDK_CAM_GEMM_SWAP=1/0 forces the choice.
+    bool rows_n = cam_grouped_gemm_rows_n_pays(num_experts, rows_per_expert_hint, n_dim, k_dim, mode) != 0;
+    if (sw_swap >= 0) rows_n = sw_swap == 1;
+    rows_n = rows_n && ue8m0 && !pair && p.bulk_push != 0;
     // The combine-send epilogue of the block-scaled kernels overlaps converting a half tile with the copies of the previous
     // one (two staging buffers, paid for with pipeline stages); UMDK_CAM_GEMM_STAGING2=0 keeps the one-buffer form.
     // On by default in the CTA-pair kernel only: the one-CTA kernel, used for small experts, lives on streaming weights
@@ -1068,7 +1085,7 @@ extern "C" int cam_grouped_gemm_mxfp8(CamBuffer* b, const void* a_q, const float
 static int grouped_gemm_w8a8_impl(CamBuffer* b, const void* a_q, const float* a_scales, int a_rows, const void* w_q,
                                   const float* w_scales, const int* expert_offsets, int num_experts, int n_dim,
                                   int k_dim, int mode, void* out_bf16, float* act_f32, float* row_amax,
-                                  const int* row_src, int topk, cudaStream_t stream) {
+                                  const int* row_src, int topk, int rows_per_expert_hint, cudaStream_t stream) {
     CAM_CHECK(a_q && a_scales && w_q && w_scales && expert_offsets, "grouped_gemm_w8a8: null operand");
     CAM_CHECK(num_experts >= 1 && a_rows >= 1, "grouped_gemm_w8a8: empty problem");
     CAM_CHECK(k_dim >= 128 && k_dim % 128 == 0, "grouped_gemm_w8a8: K %d must be a multiple of 128", k_dim);
@@ -1087,10 +1104,6 @@ static int grouped_gemm_w8a8_impl(CamBuffer* b, const void* a_q, const float* a_
     } else {
         CAM_CUDA(cudaGetDevice(&device));
     }
-    CUtensorMap ta, tb;
-    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows), cam_grouped_gemm_rows_n_box()) != 0)
-        return -1;
-    if (make_tmap(b, &tb, w_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(num_experts) * n_dim) != 0) return -1;
     cam::GroupedGemmParams p{};
     p.expert_offsets = expert_offsets;
     p.num_experts = num_experts;
@@ -1133,7 +1146,16 @@ static int grouped_gemm_w8a8_impl(CamBuffer* b, const void* a_q, const float* a_
     }
     int sms = 0;
     CAM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int rc = cam_launch_grouped_gemm_w8a8_rows_n(&p, &ta, &tb, sms, stream);
+    bool rows_n = cam_grouped_gemm_rows_n_pays(num_experts, rows_per_expert_hint, n_dim, k_dim, mode) != 0;
+    const int sw_swap = b ? b->env_swap : env_now("UMDK_CAM_GEMM_SWAP");
+    if (sw_swap >= 0) rows_n = sw_swap == 1;
+    CUtensorMap ta, tb;
+    if (make_tmap(b, &ta, a_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(a_rows),
+                  rows_n ? cam_grouped_gemm_rows_n_box() : 128) != 0)
+        return -1;
+    if (make_tmap(b, &tb, w_q, static_cast<uint64_t>(k_dim), static_cast<uint64_t>(num_experts) * n_dim) != 0) return -1;
+    const int rc = rows_n ? cam_launch_grouped_gemm_w8a8_rows_n(&p, &ta, &tb, sms, stream)
+                          : cam_launch_grouped_gemm_w8a8(&p, &ta, &tb, sms, stream);
     CAM_CHECK(rc == 0, "grouped_gemm_w8a8 launch failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
     if (b != nullptr) ++b->launches;
     return 0;
@@ -1143,7 +1165,7 @@ extern "C" int cam_grouped_gemm_w8a8(const void* a_q, const float* a_scales, int
                                      const float* w_scales, const int* expert_offsets, int num_experts, int n_dim,
                                      int k_dim, void* out_bf16, cudaStream_t stream) {
     return grouped_gemm_w8a8_impl(nullptr, a_q, a_scales, a_rows, w_q, w_scales, expert_offsets, num_experts, n_dim,
-                                  k_dim, 0, out_bf16, nullptr, nullptr, nullptr, 1, stream);
+                                  k_dim, 0, out_bf16, nullptr, nullptr, nullptr, 1, num_experts > 0 ? a_rows / num_experts : 0, stream);
 }
 
 extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* expert_ids, int idx_is_i64,
@@ -1156,6 +1178,8 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
     CAM_CHECK(w1_q && w1_s && w2_q && w2_s && topk_weights && out, "fused_moe_w8a8: null operand");
     const int El = (gemm_experts > 0 && gemm_experts <= E / b->num_ranks) ? gemm_experts : E / b->num_ranks;
     const CamLayout& L = b->layout;
+    // mean rows per local expert when routing is balanced: every rank sends T * K rows in total
+    const int rows_hint = static_cast<int>(static_cast<int64_t>(T) * K * b->num_ranks / E);
     CAM_CUDA(cudaSetDevice(b->device));
     if (b->act_f32 == nullptr) {  // first use of the int8 path on this buffer
         CAM_CUDA(cudaMalloc(&b->act_f32, static_cast<size_t>(L.capacity) * L.hidden * sizeof(float)));
@@ -1176,7 +1200,7 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
         const float* recv_s = reinterpret_cast<const float*>(b->base + L.off_recv_scales);
         const int* recv_src = reinterpret_cast<const int*>(b->base + L.off_recv_src);
         if (grouped_gemm_w8a8_impl(b, recv_x, recv_s, L.capacity, w1_q, w1_s, b->expert_offsets, El, 2 * inter, h, 1,
-                                   nullptr, b->act_f32, b->row_amax, nullptr, K, stream) != 0)
+                                   nullptr, b->act_f32, b->row_amax, nullptr, K, rows_hint, stream) != 0)
             return -1;
         const int rc = cam_launch_rowquant_int8(b->act_f32, b->row_amax, b->expert_offsets, El, inter, b->act_q, b->act_s,
                                                 stream);
@@ -1184,7 +1208,7 @@ extern "C" int cam_fused_moe_w8a8(CamBuffer* b, const void* x, const void* exper
     if (b != nullptr) ++b->launches;
         stamp(2);
         if (grouped_gemm_w8a8_impl(b, b->act_q, b->act_s, L.capacity, w2_q, w2_s, b->expert_offsets, El, h, inter, 2,
-                                   nullptr, nullptr, nullptr, recv_src, K, stream) != 0)
+                                   nullptr, nullptr, nullptr, recv_src, K, rows_hint, stream) != 0)
             return -1;
     }
     stamp(3);

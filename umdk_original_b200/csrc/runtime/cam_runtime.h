@@ -147,7 +147,11 @@ int cam_fused_moe_mxfp8(CamBuffer* b, const void* x_bf16, const void* expert_ids
                         const float* w2_s, void* out_bf16, int64_t* expert_token_nums, int T, int K, int h,
                         int inter, int E, int gemm_experts, int phase_mask, cudaStream_t stream);
 
-// Exact W8A8 (kernels/rowquant_i8.cu, grouped_gemm_rows_n.cuh): int8 activations [rows, K] with one fp32 scale per row, int8
+// 1 where the rows-as-N kernel is chosen for a grouped GEMM of these sizes (mean rows per expert below the CTA pairs' line, or
+// int8), 0 where the one-CTA kernel is.
+int cam_grouped_gemm_rows_n_pays(int num_experts, int rows_per_expert, int n_dim, int k_dim, int mode);
+
+// Exact W8A8 (kernels/grouped_gemm_i8.cu, grouped_gemm_rows_n.cuh, rowquant_i8.cu): int8 activations [rows, K] with one fp32 scale per row, int8
 // weights [E, N, K] (K contiguous) with one fp32 scale per output channel [E, N], int32 accumulation.
 int cam_grouped_gemm_w8a8(const void* a_q, const float* a_scales, int a_rows, const void* w_q, const float* w_scales,
                           const int* expert_offsets, int num_experts, int n_dim, int k_dim, void* out_bf16,
