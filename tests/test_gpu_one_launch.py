@@ -102,11 +102,21 @@ def test_low_latency_pair_in_one_launch(t, h, e, k, skip, quant, wire):
 
 
 @pytest.mark.parametrize("t,e,k,r", [(0, 8, 2, 2), (1, 1, 1, 1), (33, 72, 3, 72), (4097, 256, 8, 8), (16384, 64, 16, 4),
-                                     (16385, 64, 2, 64)])  # 16384 tokens: the most the one-launch form serves
+                                     (16385, 64, 2, 64)])  # one and two launches
 def test_layout_at_its_sizes(t, e, k, r):
     idx = torch.randint(-1, e + 1, (t, k), generator=torch.Generator().manual_seed(t))
     got = ops.get_dispatch_layout(idx.to(DEV), e, r)
     for a, b in zip(got, ref.get_dispatch_layout(idx, e, r)):
+        assert torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("dtype,offset", [(torch.int64, 0), (torch.int64, 1), (torch.int32, 1)])  # ids off the 16-byte grid
+@pytest.mark.parametrize("t,e,k,r", [(4095, 63, 5, 7), (4097, 64, 8, 8), (8192, 256, 8, 8), (8193, 256, 8, 8), (8192, 256, 9, 8),
+                                     (100, 72, 8, 9), (31, 1024, 6, 4)])
+def test_layout_on_both_sides_of_its_limits(t, e, k, r, dtype, offset):
+    flat = torch.randint(-1, e + 1, (t * k + offset,), generator=torch.Generator().manual_seed(t + k)).to(dtype)
+    got = ops.get_dispatch_layout(flat.to(DEV)[offset:].view(t, k), e, r)
+    for a, b in zip(got, ref.get_dispatch_layout(flat[offset:].view(t, k), e, r)):
         assert torch.equal(a.cpu(), b)
 
 

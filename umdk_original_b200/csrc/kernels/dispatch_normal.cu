@@ -685,43 +685,77 @@ __global__ void layout_kernel(const void* topk_idx, int idx_is_i64, int T, int K
     for (int i = threadIdx.x; i < E; i += blockDim.x) if (s_exp[i]) atomicAdd(&num_tokens_per_expert[i], s_exp[i]);
 }
 
+// Zeroes the counters the kernel above adds to (one launch; a memset node in a graph costs as much as two).
+__global__ void layout_zero_kernel(int* num_tokens_per_rank, int R, int* num_tokens_per_expert, int E) {
+    for (int i = threadIdx.x; i < R; i += blockDim.x) num_tokens_per_rank[i] = 0;
+    for (int i = threadIdx.x; i < E; i += blockDim.x) num_tokens_per_expert[i] = 0;
+}
+
 // The same in ONE launch without zeroed outputs, for batches of ordinary size: a cluster of kLayoutCtas CTAs counts in
 // shared memory, and after a cluster barrier every CTA adds up its share of the counters over the cluster's shared memories.
-// The call is bound by launches (about 3 us of host time each), not by the 64 bytes per token it reads: the counting kernel
-// above needs its three outputs zeroed first.  Up to kLayoutClusterTokens (four tokens per thread) the few CTAs cost less
-// than those launches; beyond, the whole GPU counts.  4096 tokens x 8: 22.5 us -> 9.6 us per call.
-constexpr int kLayoutCtas = 8, kLayoutThreads = 512, kLayoutClusterTokens = 4 * kLayoutCtas * kLayoutThreads;
+// The call is bound by launches (2.5 us of host time each beside 6 us of allocations and dispatch), not by the 64 bytes per
+// token it reads, as long as every thread has few tokens, ids and ranks: 4096 tokens x 8 ids, 8 ranks take 9.0 us per call
+// (5.4 on the device) against 11.5 (4.6) for the two launches above, 8192 tokens 10.2 (7.5) against 11.4 (4.6).  The few CTAs
+// lose beyond that: 16384 tokens (8 ids, 8 ranks) took 16.6 us against 11.4, 4096 tokens x 16 ids 12.3 against 11.4, 64 ranks 33
+// against 21.  (Three fills and the kernel: 22 to 27 us.)
+constexpr int kLayoutCtas = 8, kLayoutThreads = 512, kLayoutClusterTokens = 2 * kLayoutCtas * kLayoutThreads;
+constexpr int kLayoutClusterIds = 8, kLayoutClusterRanks = 8;
 
 __global__ void __cluster_dims__(kLayoutCtas, 1, 1) __launch_bounds__(kLayoutThreads)
 layout_cluster_kernel(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R, int* num_tokens_per_rank,
                       int* num_tokens_per_expert, uint8_t* is_token_in_rank) {
-    __shared__ int s_cnt[CAM_MAX_EXPERTS + CAM_MAX_RANKS];  // per expert, then per rank
+    __shared__ int s_cnt[CAM_MAX_EXPERTS + kLayoutClusterRanks];  // per expert, then per rank
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = static_cast<int>(threadIdx.x), rank = static_cast<int>(cluster.block_rank());
     const int n = E + R, El = E / R;
+    // two 64-bit ids per load where rows allow it: 8 ids per token are 64 bytes, a cache line for every other lane
+    const bool pairs = idx_is_i64 && (K & 1) == 0 && (reinterpret_cast<uintptr_t>(topk_idx) & 15u) == 0u;
+    int id[2][kLayoutClusterIds];  // both tokens' ids are in flight before the first is counted
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int t = (u * kLayoutCtas + rank) * kLayoutThreads + tid;
+        if (pairs) {
+#pragma unroll
+            for (int k = 0; k < kLayoutClusterIds; k += 2) {
+                const longlong2 v = (t < T && k < K) ? __ldg(reinterpret_cast<const longlong2*>(topk_idx) +
+                                                             (static_cast<size_t>(t) * K + k) / 2)
+                                                     : make_longlong2(-1, -1);
+                id[u][k] = (v.x >= 0 && v.x < E) ? static_cast<int>(v.x) : -1;
+                id[u][k + 1] = (v.y >= 0 && v.y < E) ? static_cast<int>(v.y) : -1;
+            }
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < kLayoutClusterIds; ++k)
+            id[u][k] = (t < T && k < K) ? load_expert_id(topk_idx, idx_is_i64, static_cast<size_t>(t) * K + k) : -1;
+    }
     for (int i = tid; i < n; i += kLayoutThreads) s_cnt[i] = 0;
     __syncthreads();
-    for (int tb = rank * kLayoutThreads + (tid & ~31); tb < T; tb += kLayoutCtas * kLayoutThreads) {
-        const int t = tb + (tid & 31);  // whole warps stay together: the last one may hold lanes past T
-        unsigned long long seen_lo = 0ull, seen_hi = 0ull;  // ranks 0..63 and 64..127
-        for (int k0 = 0; k0 < K; k0 += 8) {                 // eight loads in flight
-            int id[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                id[j] = (t < T && k0 + j < K) ? load_expert_id(topk_idx, idx_is_i64, static_cast<size_t>(t) * K + k0 + j) : -1;
+    for (int u = 0; u < 2; ++u) {
+        const int t = (u * kLayoutCtas + rank) * kLayoutThreads + tid;  // whole warps stay together: some lanes may be past T
+        if (t - (tid & 31) >= T) break;
+        uint32_t seen = 0u;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (id[j] < 0 || id[j] >= E) continue;
-                atomicAdd(&s_cnt[id[j]], 1);
-                const int r = id[j] / El;
-                if (r < 64) seen_lo |= 1ull << r; else seen_hi |= 1ull << (r - 64);
-            }
+        for (int k = 0; k < kLayoutClusterIds; ++k) {
+            if (id[u][k] < 0 || id[u][k] >= E) continue;
+            atomicAdd(&s_cnt[id[u][k]], 1);
+            seen |= 1u << (id[u][k] / El);
         }
         for (int r = 0; r < R; ++r) {
-            const bool in = (r < 64) ? ((seen_lo >> r) & 1ull) : ((seen_hi >> (r - 64)) & 1ull);
-            if (t < T) is_token_in_rank[static_cast<size_t>(t) * R + r] = in ? 1 : 0;
+            const bool in = (seen >> r) & 1u;
+            if (t < T && R != 8) is_token_in_rank[static_cast<size_t>(t) * R + r] = in ? 1 : 0;
             const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);  // one atomic per warp: few ranks, many tokens
             if ((tid & 31) == 0 && all != 0u) atomicAdd(&s_cnt[E + r], __popc(all));
+        }
+        if (t < T && R == 8) {  // bit r of `seen` into byte r: one store instead of eight
+            uint32_t lo = 0u, hi = 0u;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                lo |= ((seen >> r) & 1u) << (8 * r);
+                hi |= ((seen >> (r + 4)) & 1u) << (8 * r);
+            }
+            *reinterpret_cast<uint2*>(is_token_in_rank + static_cast<size_t>(t) * 8) = make_uint2(lo, hi);
         }
     }
     cluster.sync();
@@ -762,14 +796,13 @@ extern "C" int cam_launch_dispatch_normal(const cam::DispatchNormalParams* p, in
 extern "C" int cam_launch_layout(const void* topk_idx, int idx_is_i64, int T, int K, int E, int R,
                                  int* num_tokens_per_rank, int* num_tokens_per_expert,
                                  uint8_t* is_token_in_rank, cudaStream_t stream) {
-    if (T <= cam::kLayoutClusterTokens) {
+    const bool aligned = (reinterpret_cast<uintptr_t>(is_token_in_rank) & 7u) == 0u;  // eight ranks' bytes in one store
+    if (T <= cam::kLayoutClusterTokens && K <= cam::kLayoutClusterIds && R <= cam::kLayoutClusterRanks && aligned) {
         cam::layout_cluster_kernel<<<cam::kLayoutCtas, cam::kLayoutThreads, 0, stream>>>(
             topk_idx, idx_is_i64, T, K, E, R, num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank);
         return static_cast<int>(cudaGetLastError());
     }
-    cudaError_t e = cudaMemsetAsync(num_tokens_per_rank, 0, sizeof(int) * R, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(num_tokens_per_expert, 0, sizeof(int) * E, stream);
-    if (e != cudaSuccess) return static_cast<int>(e);
+    cam::layout_zero_kernel<<<1, 512, 0, stream>>>(num_tokens_per_rank, R, num_tokens_per_expert, E);
     const int threads = 256;
     int blocks = (T + threads - 1) / threads;
     const int cap = 4 * cam::sm_count_of_current_device();  // the kernel strides over the tokens
