@@ -30,10 +30,12 @@ namespace cam {
 constexpr int kLLThreads = 512;
 constexpr int kLLWarps = kLLThreads / 32;
 constexpr int kLLGroups = kLLThreads / 128;  // the int8 form quantises one row per group of four warps
-// A group of one rank with at most this many pairs finds the slots of the pairs it handles by scanning the ids: 2048 ids
-// are 64 steps of a warp, about a microsecond; with more, every CTA has several tokens and scans as often, and the chunk x
-// expert table of the general kernel, built once per CTA, is the cheaper way.
-constexpr int kLLScanPairs = 2048;
+// A group of one rank with at most this many pairs finds the slots of the pairs it handles by scanning the ids: 8192 ids are 256
+// steps of a warp.  Against the general kernel, which exchanges slabs and cells with itself (device time, one B200; rows of
+// 7168, 256 experts, top-8, bf16 / int8 / e4m3): 2048 pairs 13 / 22 / 11 us against 32 / 36 / 26, 4096 pairs 24 / 39 / 20 against
+// 56 / 61 / 41, 8192 pairs 49 / 94 / 42 against 147 / 163 / 121; rows of 2048, 64 experts, top-4, 4096 pairs 20 / 27 / 22 against
+// 31 / 36 / 32.  More pairs were not measured and take the general kernel.
+constexpr int kLLScanPairs = 8192;
 
 __device__ __forceinline__ void ll_record_status(CamStatus* st, int code, int who, int detail) {
     if (atomicCAS(&st->code, 0, code) == 0) {
