@@ -5,6 +5,7 @@ import torch
 
 import umdk_original_b200 as u
 from umdk_original_b200.ops import reference as ref
+from umdk_original_b200.parallel import PHASE_RECV, PHASE_SEND, run_virtual
 
 pytestmark = pytest.mark.gpu
 ops = torch.ops.umdk_cam_op_lib
@@ -47,3 +48,24 @@ def test_low_latency_batch_that_does_not_fit():
     ops.get_dispatch_layout(torch.zeros(4, 2, dtype=torch.int64, device=DEV), 16, 1)
     _low_latency(buf, 8, 128, 16, 8, 0, seed=1)
     buf.destroy()
+
+
+def test_low_latency_rows_past_the_outputs_are_reported():
+    # rank 0 has 2 tokens, so its outputs hold 2 x 2 rows; rank 1 sends it 8 more than that
+    tokens, e, h = (2, 8), 2, 128
+    bufs = u.Buffer.virtual(2, u.CamConfig(num_experts=e, max_tokens=8, hidden=h, topk=1, ll_max_tokens=8, timeout_ms=2000.0),
+                            DEV, name="past_")
+    x = [torch.randn(t, h, generator=torch.Generator().manual_seed(t)).to(torch.bfloat16) for t in tokens]
+    idx = [torch.zeros(t, 1, dtype=torch.int32, device=DEV) for t in tokens]
+
+    def disp(r):
+        return ops.moe_dispatch_shmem(x[r].to(DEV), idx[r], None, None, 2, r, e, 1, 0, 0, 0, 0, 0, 0, 1, bufs[r].handle)
+
+    res = run_virtual(disp, 2, masks=(PHASE_SEND, PHASE_RECV))
+    assert res[0][0].shape[0] == 4 and torch.equal(res[0][0].cpu(), torch.cat(x)[:4])
+    with pytest.raises(u.CamError) as ei:
+        bufs[0].check()
+    assert ei.value.who == 5 and ei.value.detail == 10  # the rows there were
+    bufs[1].check()
+    for b in bufs:
+        b.destroy()

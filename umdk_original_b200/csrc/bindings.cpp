@@ -533,7 +533,7 @@ std::vector<at::Tensor> moe_dispatch_shmem_bf16(const at::Tensor& x, const at::T
                            static_cast<int>(K), static_cast<int>(h), static_cast<int>(E),
                            static_cast<int>(active), static_cast<int>(quantMode), static_cast<int>(expertTokenNumsType),
                            expandX.data_ptr(), dynScales.data_ptr<float>(), expandIdx.data_ptr<int>(),
-                           expandSrc.data_ptr<int>(), tokenNums.data_ptr<int64_t>(), epSend.data_ptr<int>(),
+                           expandSrc.data_ptr<int>(), static_cast<int>(A1), tokenNums.data_ptr<int64_t>(), epSend.data_ptr<int>(),
                            total.data_ptr<int>(), tpSend.data_ptr<int>(), static_cast<int>(tpSend.numel()),
                            (g_phase_mask & 7) & (CAM_PHASE_SEND | CAM_PHASE_RECV), b->stream()));
     if (launches) {

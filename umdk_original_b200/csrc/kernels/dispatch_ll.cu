@@ -62,7 +62,6 @@ __device__ void dispatch_ll_one_rank(const DispatchLLParams& p, uint8_t* dyn_sme
     int* s_ids = reinterpret_cast<int*>(dyn_smem);
     int* s_slot = s_ids + npairs;
     uint8_t* stage0 = dyn_smem + ((static_cast<size_t>(npairs) * 8 + 15) & ~static_cast<size_t>(15));
-    const int max_out = p.T * min(E, K);  // rows the outputs hold
 
     trace_point(p.trace, 0);
     for (int e = tid; e < E; e += kLLThreads) s_run[e] = 0;
@@ -88,7 +87,7 @@ __device__ void dispatch_ll_one_rank(const DispatchLLParams& p, uint8_t* dyn_sme
             p.ep_send_counts[e] = s_cum[e];
             p.expert_token_nums[e] = static_cast<long long>(p.count_type == 1 ? s_run[e] : s_cum[e]);
         }
-        if (tid == 0) p.total_rows[0] = s_cum[E - 1];
+        if (tid == 0) p.total_rows[0] = min(s_cum[E - 1], p.max_out);
     }
     trace_point(p.trace, 1);
     // output row of pair i, or -1
@@ -96,7 +95,7 @@ __device__ void dispatch_ll_one_rank(const DispatchLLParams& p, uint8_t* dyn_sme
         const int e = s_ids[i];
         if (e < 0 || slot >= p.max_tokens) return -1;
         const int r = s_cum[e] - s_run[e] + slot;
-        if (r < max_out) return r;
+        if (r < p.max_out) return r;
         if (lane == 0) ll_record_status(p.status, CAM_ERR_BAD_INDEX, 5, r);
         return -1;
     };
@@ -412,11 +411,14 @@ __global__ void __launch_bounds__(kLLThreads, 1) dispatch_ll_kernel(const Dispat
                 p.expert_token_nums[le] = (p.count_type == 1) ? static_cast<long long>(end - begin)
                                                               : static_cast<long long>(end);
             }
-            if (tid == 0) p.total_rows[0] = s_cum[E - 1];
+            if (tid == 0) p.total_rows[0] = min(s_cum[E - 1], p.max_out);
         }
         // pack the slabs into the contiguous output: output row r belongs to the cell o with
-        // s_cum[o-1] <= r < s_cum[o]
-        const int total = s_cum[E - 1];
+        // s_cum[o-1] <= r < s_cum[o].  The outputs are sized for this rank's token count and distinct experts per token; a rank
+        // that sends more tokens, or names an expert twice, can go past them.
+        const int total = min(s_cum[E - 1], p.max_out);
+        if (s_cum[E - 1] > p.max_out && blockIdx.x == 0 && tid == 0)
+            ll_record_status(p.status, CAM_ERR_BAD_INDEX, 5, s_cum[E - 1]);
         for (int r = gwarp; r < total; r += nwarps) {
             int lo = 0, hi = E - 1;
             while (lo < hi) {

@@ -120,6 +120,7 @@ struct DispatchLLParams {
     int64_t* expert_token_nums;  // [E_local]
     int* ep_send_counts;      // [E_local*R] inclusive cumsum
     int* total_rows;          // [1]
+    int max_out;              // rows that expand_x, expand_scales and expand_src hold: a row past them is reported, not written
     int* tp_zero;             // [tp_words] set to zero (the counts of the tensor-parallel exchange, which may follow)
     int tp_words;
     CamStatus* status;

@@ -812,7 +812,7 @@ extern "C" int cam_combine(CamBuffer* b, const void* y, const int* row_src, cons
 extern "C" int cam_dispatch_ll(CamBuffer* b, const void* x, const void* expert_ids, int idx_is_i64,
                                const float* smooth, int T, int K, int h, int E, int active_tokens, int quant_mode,
                                int count_type, void* expand_x, float* expand_scales, int* expand_idx,
-                               int* expand_src, int64_t* expert_token_nums, int* ep_send_counts, int* total_rows,
+                               int* expand_src, int max_out, int64_t* expert_token_nums, int* ep_send_counts, int* total_rows,
                                int* tp_zero, int tp_words, int phase_mask, cudaStream_t stream) {
     if (check_common(b, T, K, h, E, "dispatch_ll") != 0) return -1;
     CAM_CHECK(b->layout.ll_max_tokens > 0, "dispatch_ll: the buffer was created without low-latency regions");
@@ -851,6 +851,7 @@ extern "C" int cam_dispatch_ll(CamBuffer* b, const void* x, const void* expert_i
     p.expert_token_nums = expert_token_nums;
     p.ep_send_counts = ep_send_counts;
     p.total_rows = total_rows;
+    p.max_out = max_out;
     p.tp_zero = tp_zero;
     p.tp_words = tp_words;
     p.status = b->d_status;

@@ -109,11 +109,12 @@ int cam_combine(CamBuffer* b, const void* y_bf16, const int* row_src, const int*
                 const void* topk_idx, int idx_is_i64, const float* topk_weights, void* out_bf16, int T, int K, int h, int E,
                 int low_latency, int comm_quant, int phase_mask, cudaStream_t stream);
 
+// The outputs hold max_out rows; rows past them are not written, and the status says how many there were.
 // total_rows ends as 0 when the call receives nothing (phase_mask without RECV, or a timed-out wait); the tp_words words
 // at tp_zero (may be null with 0 words) are set to zero.
 int cam_dispatch_ll(CamBuffer* b, const void* x_bf16, const void* expert_ids, int idx_is_i64, const float* smooth,
                     int T, int K, int h, int E, int active_tokens, int quant_mode, int count_type,
-                    void* expand_x, float* expand_scales, int* expand_idx, int* expand_src,
+                    void* expand_x, float* expand_scales, int* expand_idx, int* expand_src, int max_out,
                     int64_t* expert_token_nums, int* ep_send_counts, int* total_rows, int* tp_zero, int tp_words,
                     int phase_mask, cudaStream_t stream);
 
