@@ -45,7 +45,8 @@ def _one_launch_between(fn):
     return out0, out1
 
 
-@pytest.mark.parametrize("t,h,e,k,wire", [(1, 128, 2, 1, 0), (37, 640, 8, 3, 0), (37, 640, 8, 3, 2), (90, 1152, 16, 8, 2),
+@pytest.mark.parametrize("t,h,e,k,wire", [(1, 128, 2, 1, 0), (37, 640, 8, 3, 0), (37, 640, 8, 3, 2), (37, 2176, 8, 3, 2),
+                                          (90, 4224, 16, 8, 2), (90, 1152, 16, 8, 2),
                                           (200, 256, 32, 12, 0), (200, 256, 32, 12, 2)])
 def test_low_latency_combine(t, h, e, k, wire):
     bufs = u.Buffer.virtual(2, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, ll_max_tokens=t, timeout_ms=2000.0),

@@ -61,9 +61,11 @@ def test_prefill_pair_in_one_launch(t, h, e, k, skip):
 
 
 @pytest.mark.parametrize("quant,wire", [(0, 0), (2, 2), (3, 2), (4, 0)])
-@pytest.mark.parametrize("t,h,e,k,skip", [(1, 128, 1, 1, 0), (5, 1152, 6, 3, 2), (151, 512, 64, 8, 5), (256, 128, 8, 8, 0),
+@pytest.mark.parametrize("t,h,e,k,skip", [(1, 128, 1, 1, 0), (5, 1152, 6, 3, 2), (35, 2176, 16, 3, 4), (40, 4224, 32, 8, 3),
+                                          (40, 4096, 32, 9, 3), (151, 512, 64, 8, 5), (256, 128, 8, 8, 0),
                                           (257, 128, 16, 8, 3), (1024, 128, 64, 8, 5),
-                                          (1025, 128, 64, 8, 7)])  # 8192 pairs: the most the scan of the ids serves
+                                          (1025, 128, 64, 8, 7)])
+# 8192 pairs: the most the scan of the ids serves; int8 rows of more than 2048 and at least 512 x k: combined in place
 def test_low_latency_pair_in_one_launch(t, h, e, k, skip, quant, wire):
     buf = u.Buffer(None, u.CamConfig(num_experts=e, max_tokens=t, hidden=h, topk=k, ll_max_tokens=t, timeout_ms=2000.0),
                    device=DEV, rank=0, num_ranks=1)

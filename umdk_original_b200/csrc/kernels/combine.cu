@@ -64,8 +64,13 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
     // layer's reduce, whose rows the GEMM epilogue has pushed, and the phase-by-phase harness) uses the slots.
     // Bound by memory traffic: 4096 tokens x 8 rows of 14 KB on one GPU took 263 us with every row copied to its slot first
     // (1.47 GB moved), 102 us with the rows gathered in place (0.53 GB, 5.2 TB/s).
+    // With int8 rows the gathering warp quantises its 512-element slices of K rows one after the other, where the push
+    // quantises every row in a warp of its own: in place only if that is no more than a row, and a long one (one rank, 64
+    // tokens, pushed and in place: 7168 x top-8 24.7 and 18.9 us, 4096 x 8 21.4 and 19.3, 2048 x 4 15.5 and 16.2, 2048 x 12 20.5
+    // and 22.6, 1024 x 9 16.5 and 19.5).
     const bool in_place = p.local_row != nullptr && p.y != nullptr &&
-                          (p.phase_mask & (CAM_PHASE_SEND | CAM_PHASE_RECV)) == (CAM_PHASE_SEND | CAM_PHASE_RECV);
+                          (p.phase_mask & (CAM_PHASE_SEND | CAM_PHASE_RECV)) == (CAM_PHASE_SEND | CAM_PHASE_RECV) &&
+                          (p.comm_quant != 2 || (p.K * 512 <= p.h && p.h > 2048));
     if (tid == 0) s_abort = 0u;
     __syncthreads();
 
@@ -231,41 +236,58 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                     float acc[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-                    for (int k = 0; k < p.K; ++k) {
-                        if (!((valid >> k) & 1u)) continue;
-                        const uint64_t from = s_row[warp][k];
-                        if (from & 1ull) {
-                            // a row of y: quantised to the wire format here (8 lanes hold a 128-element block), so that
-                            // a row counts the same whether it travelled or not
-                            const uint8_t* yrow = reinterpret_cast<const uint8_t*>(from & ~1ull) + static_cast<size_t>(c) * 2;
-                            const uint4 y0 = ld_cg_v4(yrow), y1 = ld_cg_v4(yrow + 16);
-                            const float f[16] = {bf16_lo(y0.x), bf16_hi(y0.x), bf16_lo(y0.y), bf16_hi(y0.y),
-                                                 bf16_lo(y0.z), bf16_hi(y0.z), bf16_lo(y0.w), bf16_hi(y0.w),
-                                                 bf16_lo(y1.x), bf16_hi(y1.x), bf16_lo(y1.y), bf16_hi(y1.y),
-                                                 bf16_lo(y1.z), bf16_hi(y1.z), bf16_lo(y1.w), bf16_hi(y1.w)};
-                            float amax = 0.f;
+                    for (int k0 = 0; k0 < p.K; k0 += 4) {  // the loads of four rows are in flight before the first is added
+                        uint4 v0[4], v1[4];
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-                            const uint32_t group = 0xFFu << (lane & 24u);  // h is a multiple of 128: all 8 lanes are here
-#pragma unroll
-                            for (int sft = 4; sft >= 1; sft >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, sft));
-                            const float a = fmaxf(amax, 1e-12f);
-                            const float inv = 127.f / a;
-                            const float sc = (a / 127.f) * s_w[warp][k];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                acc[j] = fmaf(sc, static_cast<float>(static_cast<int>(static_cast<int8_t>(
-                                                      static_cast<uint32_t>(__float2int_rn(f[j] * inv)) & 0xFFu))), acc[j]);
-                            continue;
+                        for (int u = 0; u < 4; ++u) {
+                            const int k = k0 + u;
+                            v0[u] = v1[u] = make_uint4(0, 0, 0, 0);
+                            if (k >= p.K || !((valid >> k) & 1u)) continue;
+                            const uint64_t from = s_row[warp][k];
+                            if (from & 1ull) {
+                                const uint8_t* yrow = reinterpret_cast<const uint8_t*>(from & ~1ull) + static_cast<size_t>(c) * 2;
+                                v0[u] = ld_cg_v4(yrow);
+                                v1[u] = ld_cg_v4(yrow + 16);
+                            } else {
+                                const uint8_t* krow = reinterpret_cast<const uint8_t*>(from);
+                                v0[u] = ld_cg_v4(krow + c);
+                                v1[u].x = __float_as_uint(__ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7)));
+                            }
                         }
-                        const uint8_t* krow = reinterpret_cast<const uint8_t*>(from);
-                        const uint4 q = ld_cg_v4(krow + c);
-                        const float sc = __ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7)) * s_w[warp][k];
-                        const uint32_t wq[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int b8 = static_cast<int>(static_cast<int8_t>((wq[j >> 2] >> (8 * (j & 3))) & 0xFFu));
-                            acc[j] = fmaf(sc, static_cast<float>(b8), acc[j]);
+                        for (int u = 0; u < 4; ++u) {
+                            const int k = k0 + u;
+                            if (k >= p.K || !((valid >> k) & 1u)) continue;
+                            if (s_row[warp][k] & 1ull) {
+                                // a row of y: quantised to the wire format here (8 lanes hold a 128-element block), so that
+                                // a row counts the same whether it travelled or not
+                                const uint4 y0 = v0[u], y1 = v1[u];
+                                const float f[16] = {bf16_lo(y0.x), bf16_hi(y0.x), bf16_lo(y0.y), bf16_hi(y0.y),
+                                                     bf16_lo(y0.z), bf16_hi(y0.z), bf16_lo(y0.w), bf16_hi(y0.w),
+                                                     bf16_lo(y1.x), bf16_hi(y1.x), bf16_lo(y1.y), bf16_hi(y1.y),
+                                                     bf16_lo(y1.z), bf16_hi(y1.z), bf16_lo(y1.w), bf16_hi(y1.w)};
+                                float amax = 0.f;
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+                                const uint32_t group = 0xFFu << (lane & 24u);  // h is a multiple of 128: all 8 lanes are here
+#pragma unroll
+                                for (int sft = 4; sft >= 1; sft >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, sft));
+                                const float a = fmaxf(amax, 1e-12f);
+                                const float inv = 127.f / a;
+                                const float sc = (a / 127.f) * s_w[warp][k];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    acc[j] = fmaf(sc, static_cast<float>(static_cast<int>(static_cast<int8_t>(
+                                                          static_cast<uint32_t>(__float2int_rn(f[j] * inv)) & 0xFFu))), acc[j]);
+                                continue;
+                            }
+                            const float sc = __uint_as_float(v1[u].x) * s_w[warp][k];
+                            const uint32_t wq[4] = {v0[u].x, v0[u].y, v0[u].z, v0[u].w};
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const int b8 = static_cast<int>(static_cast<int8_t>((wq[j >> 2] >> (8 * (j & 3))) & 0xFFu));
+                                acc[j] = fmaf(sc, static_cast<float>(b8), acc[j]);
+                            }
                         }
                     }
                     uint4 r0, r1;
