@@ -46,6 +46,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&t);
 }
 
+// INT8_WIRE: comm_quant 2.  IN_PLACE: rows whose origin is this rank do not move; one launch sends and reduces.  Kernels of their
+// own, so that no form takes part in the register allocation of another (int8 with both ways of its rows in one kernel: 16 tokens
+// x 2 of 1024, pushed, 12.9 us against 12.0).
+template <bool INT8_WIRE, bool IN_PLACE>
 __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineParams p) {
     __shared__ uint32_t s_abort;
     __shared__ float s_w[kCombWarps][CAM_MAX_TOPK];
@@ -60,17 +64,10 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
     const uint32_t ep_send = p.epochs[0] + 1u, ep_recv = p.epochs[1] + 1u;
     // Rows whose origin is this rank do not move when one launch sends and reduces: the send phase notes {epoch, row}
     // per (token, k) pair, 8 bytes instead of a row written and read again, and the reduce gathers straight from y.
-    // The epoch tells this launch's entries from those of earlier ones.  A launch that runs one phase only (the fused
-    // layer's reduce, whose rows the GEMM epilogue has pushed, and the phase-by-phase harness) uses the slots.
+    // The epoch tells this launch's entries from those of earlier ones.
     // Bound by memory traffic: 4096 tokens x 8 rows of 14 KB on one GPU took 263 us with every row copied to its slot first
     // (1.47 GB moved), 102 us with the rows gathered in place (0.53 GB, 5.2 TB/s).
-    // With int8 rows the gathering warp quantises its 512-element slices of K rows one after the other, where the push
-    // quantises every row in a warp of its own: in place only if that is no more than a row, and a long one (one rank, 64
-    // tokens, pushed and in place: 7168 x top-8 24.7 and 18.9 us, 4096 x 8 21.4 and 19.3, 2048 x 4 15.5 and 16.2, 2048 x 12 20.5
-    // and 22.6, 1024 x 9 16.5 and 19.5).
-    const bool in_place = p.local_row != nullptr && p.y != nullptr &&
-                          (p.phase_mask & (CAM_PHASE_SEND | CAM_PHASE_RECV)) == (CAM_PHASE_SEND | CAM_PHASE_RECV) &&
-                          (p.comm_quant != 2 || (p.K * 512 <= p.h && p.h > 2048));
+    constexpr bool in_place = IN_PLACE;
     if (tid == 0) s_abort = 0u;
     __syncthreads();
 
@@ -109,7 +106,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
             const uint8_t* s = reinterpret_cast<const uint8_t*>(p.y) + static_cast<size_t>(i) * row_bytes;
             uint8_t* d = p.peer_base[src] + p.off_combine_buf +
                          (static_cast<size_t>(t) * p.K + k) * static_cast<size_t>(row_bytes);
-            if (p.comm_quant == 2) {
+            if constexpr (INT8_WIRE) {
                 // int8 on the wire: lane owns 8 elements per step of 256, 16 lanes share a 128-element block
                 float* dscale = reinterpret_cast<float*>(d + p.h);
                 for (int base = 0; base < p.h; base += 1024) {
@@ -221,7 +218,7 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
             __syncwarp();
             return valid;
         };
-        if (p.comm_quant == 2) {
+        if constexpr (INT8_WIRE) {
             // rows arrived as int8 + one scale per 128 elements; a lane reduces 16 elements per step
             const int chunks_q = (p.h + 511) / 512;
             const int nsplit_q = min(chunks_q, max(1, nwarps / max(p.T, 1)));
@@ -236,58 +233,76 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                     float acc[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-                    for (int k0 = 0; k0 < p.K; k0 += 4) {  // the loads of four rows are in flight before the first is added
-                        uint4 v0[4], v1[4];
+                    auto add_wire_row = [&](const uint4& q, float sc) {
+                        const uint32_t wq[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int b8 = static_cast<int>(static_cast<int8_t>((wq[j >> 2] >> (8 * (j & 3))) & 0xFFu));
+                            acc[j] = fmaf(sc, static_cast<float>(b8), acc[j]);
+                        }
+                    };
+                    // rows from the slots: the loads of four are in flight before the first is added
+                    for (int k0 = 0; !in_place && k0 < p.K; k0 += 4) {
+                        uint4 q[4];
+                        float sc[4];
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             const int k = k0 + u;
-                            v0[u] = v1[u] = make_uint4(0, 0, 0, 0);
                             if (k >= p.K || !((valid >> k) & 1u)) continue;
-                            const uint64_t from = s_row[warp][k];
-                            if (from & 1ull) {
-                                const uint8_t* yrow = reinterpret_cast<const uint8_t*>(from & ~1ull) + static_cast<size_t>(c) * 2;
-                                v0[u] = ld_cg_v4(yrow);
-                                v1[u] = ld_cg_v4(yrow + 16);
-                            } else {
-                                const uint8_t* krow = reinterpret_cast<const uint8_t*>(from);
-                                v0[u] = ld_cg_v4(krow + c);
-                                v1[u].x = __float_as_uint(__ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7)));
-                            }
+                            const uint8_t* krow = reinterpret_cast<const uint8_t*>(s_row[warp][k]);
+                            q[u] = ld_cg_v4(krow + c);
+                            sc[u] = __ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7));
                         }
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             const int k = k0 + u;
                             if (k >= p.K || !((valid >> k) & 1u)) continue;
-                            if (s_row[warp][k] & 1ull) {
-                                // a row of y: quantised to the wire format here (8 lanes hold a 128-element block), so that
-                                // a row counts the same whether it travelled or not
-                                const uint4 y0 = v0[u], y1 = v1[u];
-                                const float f[16] = {bf16_lo(y0.x), bf16_hi(y0.x), bf16_lo(y0.y), bf16_hi(y0.y),
-                                                     bf16_lo(y0.z), bf16_hi(y0.z), bf16_lo(y0.w), bf16_hi(y0.w),
-                                                     bf16_lo(y1.x), bf16_hi(y1.x), bf16_lo(y1.y), bf16_hi(y1.y),
-                                                     bf16_lo(y1.z), bf16_hi(y1.z), bf16_lo(y1.w), bf16_hi(y1.w)};
-                                float amax = 0.f;
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-                                const uint32_t group = 0xFFu << (lane & 24u);  // h is a multiple of 128: all 8 lanes are here
-#pragma unroll
-                                for (int sft = 4; sft >= 1; sft >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, sft));
-                                const float a = fmaxf(amax, 1e-12f);
-                                const float inv = 127.f / a;
-                                const float sc = (a / 127.f) * s_w[warp][k];
-#pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    acc[j] = fmaf(sc, static_cast<float>(static_cast<int>(static_cast<int8_t>(
-                                                          static_cast<uint32_t>(__float2int_rn(f[j] * inv)) & 0xFFu))), acc[j]);
+                            add_wire_row(q[u], sc[u] * s_w[warp][k]);
+                        }
+                    }
+                    if constexpr (IN_PLACE) {  // the next row's loads are in flight while a row is quantised
+                        uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
+                        auto fetch = [&](int k) {  // a row of y as it is, a row from the slots with its scale in n1.x
+                            if (k >= p.K || !((valid >> k) & 1u)) return;
+                            const uint64_t from = s_row[warp][k];
+                            if (from & 1ull) {
+                                const uint8_t* yrow = reinterpret_cast<const uint8_t*>(from & ~1ull) + static_cast<size_t>(c) * 2;
+                                n0 = ld_cg_v4(yrow);
+                                n1 = ld_cg_v4(yrow + 16);
+                            } else {
+                                const uint8_t* krow = reinterpret_cast<const uint8_t*>(from);
+                                n0 = ld_cg_v4(krow + c);
+                                n1.x = __float_as_uint(__ldcg(reinterpret_cast<const float*>(krow + p.h) + (c >> 7)));
+                            }
+                        };
+                        fetch(0);
+                        for (int k = 0; k < p.K; ++k) {
+                            const uint4 y0 = n0, y1 = n1;
+                            fetch(k + 1);
+                            if (!((valid >> k) & 1u)) continue;
+                            if (!(s_row[warp][k] & 1ull)) {
+                                add_wire_row(y0, __uint_as_float(y1.x) * s_w[warp][k]);
                                 continue;
                             }
-                            const float sc = __uint_as_float(v1[u].x) * s_w[warp][k];
-                            const uint32_t wq[4] = {v0[u].x, v0[u].y, v0[u].z, v0[u].w};
+                            // a row of y: quantised to the wire format here (8 lanes hold a 128-element block), so that
+                            // a row counts the same whether it travelled or not
+                            const float f[16] = {bf16_lo(y0.x), bf16_hi(y0.x), bf16_lo(y0.y), bf16_hi(y0.y),
+                                                 bf16_lo(y0.z), bf16_hi(y0.z), bf16_lo(y0.w), bf16_hi(y0.w),
+                                                 bf16_lo(y1.x), bf16_hi(y1.x), bf16_lo(y1.y), bf16_hi(y1.y),
+                                                 bf16_lo(y1.z), bf16_hi(y1.z), bf16_lo(y1.w), bf16_hi(y1.w)};
+                            float amax = 0.f;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int b8 = static_cast<int>(static_cast<int8_t>((wq[j >> 2] >> (8 * (j & 3))) & 0xFFu));
-                                acc[j] = fmaf(sc, static_cast<float>(b8), acc[j]);
-                            }
+                            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+                            const uint32_t group = 0xFFu << (lane & 24u);  // h is a multiple of 128: all 8 lanes are here
+#pragma unroll
+                            for (int sft = 4; sft >= 1; sft >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, sft));
+                            const float a = fmaxf(amax, 1e-12f);
+                            const float inv = 127.f / a;
+                            const float sc = (a / 127.f) * s_w[warp][k];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                acc[j] = fmaf(sc, static_cast<float>(static_cast<int>(static_cast<int8_t>(
+                                                      static_cast<uint32_t>(__float2int_rn(f[j] * inv)) & 0xFFu))), acc[j]);
                         }
                     }
                     uint4 r0, r1;
@@ -316,7 +331,8 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
             if (p.K <= 8) {
                 // The loads of the next 512 bytes of all rows are in flight while these are added up: with one batch at a
                 // time a warp has nothing outstanding between its last load and the store (4096 tokens x 8 rows of 14 KB:
-                // 102.6 -> 94.7 us, 5.6 TB/s).
+                // 102.6 -> 94.7 us, 5.6 TB/s).  The main loop is free of conditions: with the ends of the slice tested in it the
+                // compiler may bring the two batches back into step (102.4 us).
                 auto load8 = [&](uint4 (&v)[8], int o) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
@@ -338,10 +354,15 @@ __global__ void __launch_bounds__(kCombThreads, 1) combine_kernel(const CombineP
                 uint4 va[8], vb[8];
                 int o = o_begin + static_cast<int>(lane) * 16;
                 if (o < o_end) load8(va, o);
-                for (; o < o_end; o += 1024) {
+                for (; o + 1024 < o_end; o += 1024) {
+                    load8(vb, o + 512);
+                    add8(va, o);
+                    load8(va, o + 1024);
+                    add8(vb, o + 512);
+                }
+                if (o < o_end) {
                     if (o + 512 < o_end) load8(vb, o + 512);
                     add8(va, o);
-                    if (o + 1024 < o_end) load8(va, o + 1024);
                     if (o + 512 < o_end) add8(vb, o + 512);
                 }
                 __syncwarp();
@@ -394,6 +415,18 @@ extern "C" int cam_combine_max_grid(int device) {
 
 extern "C" int cam_launch_combine(const cam::CombineParams* p, int grid, cudaStream_t stream) {
     void* args[] = {const_cast<cam::CombineParams*>(p)};
-    return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(cam::combine_kernel), dim3(grid),
-                                                        dim3(cam::kCombThreads), args, 0, stream));
+    // A launch that runs one phase only (the fused layer's reduce, whose rows the GEMM epilogue has pushed, and the phase-by-phase
+    // harness) uses the slots.  With int8 rows the gathering warp quantises its 512-element slices of K rows one after the other,
+    // where the push quantises every row in a warp of its own: in place only if that is no more than a row, and a long one
+    // (device time, pushed and in place, one rank: 128 tokens x 8 of 7168 27.0 and 18.5 us, 61 x 6 of 5120 19.9 and 16.6, 64 x 8
+    // of 4096 19.6 and 18.2, 64 x 4 of 2048 14.3 and 15.3, 64 x 9 of 1024 14.6 and 19.7, 16 x 2 of 1024 12.0 and 13.9).
+    const bool int8 = p->comm_quant == 2;
+    const bool in_place = p->local_row != nullptr && p->y != nullptr &&
+                          (p->phase_mask & (CAM_PHASE_SEND | CAM_PHASE_RECV)) == (CAM_PHASE_SEND | CAM_PHASE_RECV) &&
+                          (!int8 || (p->K * 512 <= p->h && p->h > 2048));
+    void* const kernel = int8 ? (in_place ? reinterpret_cast<void*>(cam::combine_kernel<true, true>)
+                                          : reinterpret_cast<void*>(cam::combine_kernel<true, false>))
+                              : (in_place ? reinterpret_cast<void*>(cam::combine_kernel<false, true>)
+                                          : reinterpret_cast<void*>(cam::combine_kernel<false, false>));
+    return static_cast<int>(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(cam::kCombThreads), args, 0, stream));
 }
