@@ -51,10 +51,11 @@ constexpr uint32_t kLaunchRegs = 96, kCtrlRegs = 32, kEpiRegs = 112;
 static_assert(128 * kCtrlRegs + kEpiThreads * kEpiRegs <= kLaunchRegs * kGemmThreads,
               "setmaxnreg budget exceeds the registers the CTA owns: the kernel would hang");
 
-// Two neighbouring sums in one instruction: (a0, a1) += (s, s) * (v0, v1), each rounded as fmaf rounds it.  The epilogue warps
-// of this kernel keep the schedulers busy (0.68 instructions per cycle, the tensor pipe 32 %), and these were 64 of what a
-// warp issues per K-block.  Ragged 32-expert layer: 779 -> 765 us; what bounds the promotion after that is reading every
-// K-block's 128 KB out of tensor memory beside the MMAs.
+// Two neighbouring sums in one instruction: (a0, a1) += (s, s) * (v0, v1), each rounded as fmaf rounds it.  These were 64 of
+// what a warp issues per K-block.  Ragged 32-expert layer: 779 -> 765 us.  Nothing is saturated after that (first GEMM of 8
+// experts x 256 rows: 0.59 instructions per cycle and scheduler, 0.68 before, the tensor pipe active half of the time): the
+// stalls are spread over the loads from tensor memory, fixed latencies and barriers, as the sequence load - wait - add - load -
+// wait - add of a warp's K-block with four warps per scheduler would leave them.
 __device__ __forceinline__ void fma_pair(float& a0, float& a1, float s, uint32_t v0, uint32_t v1) {
     asm("{\n"
         ".reg .b64 a, s, v;\n"

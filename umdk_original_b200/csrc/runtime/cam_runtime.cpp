@@ -1044,8 +1044,8 @@ static int grouped_gemm_impl(CamBuffer* b, const void* a_q, const float* a_scale
     rows_n = rows_n && ue8m0 && !pair && p.bulk_push != 0;
     // The combine-send epilogue of the block-scaled kernels overlaps converting a half tile with the copies of the previous
     // one (two staging buffers, paid for with pipeline stages); UMDK_CAM_GEMM_STAGING2=0 keeps the one-buffer form.
-    // On by default in the CTA-pair kernel only: the one-CTA kernel, used for small experts, lives on streaming weights
-    // and loses more from its fourth pipeline stage than the epilogue gains (measured on one GPU, 256 experts).
+    // On by default in the CTA-pair kernel only: the one-CTA kernel lives on streaming weights and loses more with its fourth
+    // pipeline stage than the epilogue gains (measured on one GPU, 256 experts).  The rows-as-N kernel has one buffer.
     bool two_staging = mode == 2 && p.bulk_push != 0 && pair;
     if (sw_stg2 >= 0) two_staging = mode == 2 && p.bulk_push != 0 && sw_stg2 == 1;
     CUtensorMap ta, tb;
