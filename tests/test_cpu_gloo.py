@@ -281,3 +281,28 @@ def test_fp16_activations_are_accepted_and_returned_as_fp16():
     # same rows; the fp16 result is the bf16 result rounded once more
     assert (outs[torch.float16] - outs[torch.bfloat16]).abs().max() <= 1e-2 * outs[torch.bfloat16].abs().max()
     buf.destroy()
+
+
+def _shared_ranks_uneven(rank, world):
+    """Two replicas of the shared expert and 5 tokens per rank: the first replica gets 3 of every rank's."""
+    import torch
+    import umdk_original_b200 as u
+    t, h, e, k, shared = 5, 128, 4, 2, 2
+    g = torch.Generator().manual_seed(9)
+    xs = [torch.randn(t, h, generator=g).to(torch.bfloat16) for _ in range(world)]
+    idx = [torch.stack([torch.randperm(e, generator=g)[:k] for _ in range(t)]) for _ in range(world)]
+    buf = u.Buffer(None, u.CamConfig(num_experts=e * world, max_tokens=t, hidden=h, topk=k + 1, ll_max_tokens=t), name="uneven",
+                   device=torch.device("cpu"))
+    d = torch.ops.umdk_cam_op_lib.moe_dispatch_shmem(xs[rank], idx[rank], None, None, world, rank, e, 1, 0, 0, 1, shared, 0, 0, 1,
+                                                     buf.handle)
+    if rank >= shared:
+        return d[0].shape[0], int(d[3].sum())
+    mine = torch.cat([x[:3] if rank == 0 else x[3:] for x in xs])
+    assert torch.equal(d[0][:mine.shape[0]], mine)
+    return d[0].shape[0], int(d[3].sum())
+
+
+def test_low_latency_shared_ranks_with_uneven_slices():
+    res = run_gloo(_shared_ranks_uneven, 3)
+    assert {r: (st, val) for r, (st, val) in res.items()} == {
+        0: ("ok", (9, 9)), 1: ("ok", (9, 6)), 2: ("ok", (5 * 3 * 2, 5 * 3 * 2))}

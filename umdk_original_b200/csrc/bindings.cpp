@@ -494,7 +494,9 @@ std::vector<at::Tensor> moe_dispatch_shmem_bf16(const at::Tensor& x, const at::T
     const int is64 = idx_kind(ids, "expertIds");
     const int64_t K = ids.size(1);
     // rows this rank can receive (pybind/moe_dispatch_shmem.cpp:50-62)
-    const int64_t A1 = std::max<int64_t>(1, shared_rank ? (T * epWorldSize + S - 1) / S
+    // (a replica of the shared expert gets at most ceil(T / S) tokens of every rank: where S does not divide T that is more
+    // than an equal share of all tokens)
+    const int64_t A1 = std::max<int64_t>(1, shared_rank ? (T + S - 1) / S * epWorldSize
                                                         : T * epWorldSize * std::min<int64_t>(El, Kuser));
     const int64_t A = A1 * std::max<int64_t>(tpWorldSize, 1);  // with TP the partner's rows follow this rank's own
     // x_active_mask: tokens whose entry is false do not take part.  Applied on the device (no host
@@ -594,7 +596,7 @@ std::vector<at::Tensor> moe_dispatch_shmem_meta(const at::Tensor& x, const at::T
     const int64_t T = x.size(0), h = x.size(1), K = expertIds.size(1);
     const int64_t S = sharedExpertRankNum, El = moeExpertNum / (epWorldSize - S);
     const bool shared_rank = epRankId < S;
-    const int64_t A = std::max<int64_t>(1, shared_rank ? (T * epWorldSize + S - 1) / S
+    const int64_t A = std::max<int64_t>(1, shared_rank ? (T + S - 1) / S * epWorldSize
                                                        : T * epWorldSize * std::min<int64_t>(El, K));
     const at::ScalarType xdt = quantMode == 0 ? at::kBFloat16 : quantMode == 2 ? at::kChar : at::kFloat8_e4m3fn;
     if (S > 0)

@@ -143,7 +143,7 @@ def _moe_dispatch_shmem_cpu(x, expertIds, scales, xActiveMask, epWorldSize, epRa
     if sharedExpertRankNum > 0:
         ids, _, e_virtual, el = ref.remap_for_shared_ranks(expertIds, None, epWorldSize, moeExpertNum, sharedExpertRankNum)
         assert g.num_experts == e_virtual, "the Buffer must be created for R * E_local virtual experts"
-    a = max(1, -(-t * epWorldSize // sharedExpertRankNum) if shared_rank else t * epWorldSize * min(el, k))
+    a = max(1, -(-t // sharedExpertRankNum) * epWorldSize if shared_rank else t * epWorldSize * min(el, k))
     active = int(xActiveMask.sum()) if xActiveMask is not None else None
     rx, rs, src, cnt, per_e, slots = _backend().dispatch(g, x, ids, quantMode, active, scales)
     if sharedExpertRankNum > 0:
